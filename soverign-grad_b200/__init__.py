@@ -2,7 +2,8 @@
 `sovereigngrad::quantization` / `nn::QuantizedLinear*` names over torch CUDA tensors.
 
 torch is used for device memory and streams only: every computation below is a call through
-the C ABI into the hand-written sm_100a kernels.  There is no CPU path and no fallback — if the
+the C ABI into the hand-written sm_100a kernels; the calls of a token loop go through
+csrc/torch_binding.cpp, which does in native code what ctypes would.  There is no CPU path and no fallback — if the
 shared library is missing, importing this package raises.
 
 The directory name contains a hyphen, so load it with `__graft_entry__.load_package()` (which
@@ -11,6 +12,8 @@ registers it as module `sgq_b200`).
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 from dataclasses import dataclass, field
 from typing import Optional
@@ -19,6 +22,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libsgq.so")
+BINDING_PATH = os.path.join(_HERE, "lib", "_sgq_torch.so")
 
 LAYOUT_KN, LAYOUT_NK = 0, 1
 PER_TENSOR, PER_ROW = 0, 1
@@ -108,6 +112,19 @@ def _load() -> C.CDLL:
 lib = _load()
 
 
+def _load_binding():
+    """csrc/torch_binding.cpp: the hot calls below in native code (it links the libsgq.so loaded above)."""
+    if not os.path.exists(BINDING_PATH):
+        raise ImportError(f"{BINDING_PATH} is missing: build it with `python soverign-grad_b200/build.py`")
+    loader = importlib.machinery.ExtensionFileLoader("_sgq_torch", BINDING_PATH)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_sgq_torch", BINDING_PATH, loader=loader))
+    loader.exec_module(mod)
+    return mod
+
+
+_native = _load_binding()
+
+
 def check(status: int, what: str = "sgq call") -> None:
     if status != 0:
         raise SgqError(status, f"{what} failed: {lib.sgq_status_string(status).decode()}", lib.sgq_last_error().decode())
@@ -168,52 +185,27 @@ class QuantizedTensor:
         return out
 
 
+_native.set_classes(SgqError, QuantizedTensor)
+
+
 def quantize_int8(x: torch.Tensor, scheme: int = PER_ROW) -> QuantizedTensor:
     """quantization::quantize_int8 (src/quantization.cpp:11-78)."""
-    x = _f32_cuda(x)
-    shape = tuple(x.shape)
-    n = x.numel()
-    if scheme == PER_TENSOR or x.dim() < 2:            # :22
-        rows, cols, sch, nscales = 1, n, PER_TENSOR, 1
-    else:
-        rows = shape[0]
-        cols = n // rows if rows else 0
-        sch, nscales = PER_ROW, rows
-    codes = torch.empty(shape, dtype=torch.int8, device=x.device)
-    scales = torch.empty(nscales, dtype=torch.float32, device=x.device)
-    check(lib.sgq_quantize_int8(_ptr(x), rows, cols, sch, _ptr(codes), _ptr(scales), _stream()), "sgq_quantize_int8")
-    return QuantizedTensor(codes, scales, scheme, shape, n, 8)
+    return _native.quantize_int8(x, scheme)
 
 
 def quantize_int4(x: torch.Tensor, group_size: int = 32) -> QuantizedTensor:
     """quantization::quantize_int4 (src/quantization.cpp:113-159)."""
-    x = _f32_cuda(x)
-    g = 32 if group_size <= 0 else group_size
-    n = x.numel()
-    packed = torch.empty((n + 1) // 2, dtype=torch.uint8, device=x.device)
-    scales = torch.empty((n + g - 1) // g, dtype=torch.float32, device=x.device)
-    check(lib.sgq_quantize_int4(_ptr(x), n, g, _ptr(packed), _ptr(scales), _stream()), "sgq_quantize_int4")
-    return QuantizedTensor(packed, scales, PER_TENSOR, tuple(x.shape), g, 4)
+    return _native.quantize_int4(x, group_size)
 
 
 def dequantize_int8(q: QuantizedTensor) -> torch.Tensor:
     """quantization::dequantize_int8 (src/quantization.cpp:80-111)."""
-    out = torch.empty(q.original_shape, dtype=torch.float32, device=q.qdata.device)
-    n = _numel(q.original_shape)
-    per_tensor = q.scheme == PER_TENSOR or q.scales.numel() == 1       # :91
-    rows = 1 if per_tensor else q.original_shape[0]
-    cols = n // rows if rows else 0
-    check(lib.sgq_dequantize_int8(_ptr(q.qdata), _ptr(q.scales), rows, cols, PER_TENSOR if per_tensor else PER_ROW,
-                                  _ptr(out), _stream()), "sgq_dequantize_int8")
-    return out
+    return _native.dequantize(q)
 
 
 def dequantize_int4(q: QuantizedTensor) -> torch.Tensor:
     """quantization::dequantize_int4 (src/quantization.cpp:161-187)."""
-    out = torch.empty(q.original_shape, dtype=torch.float32, device=q.qdata.device)
-    check(lib.sgq_dequantize_int4(_ptr(q.qdata), _ptr(q.scales), _numel(q.original_shape), q.group_size, _ptr(out),
-                                  _stream()), "sgq_dequantize_int4")
-    return out
+    return _native.dequantize(q)
 
 
 def linear_workspace_bytes(bits: int, M: int, K: int, N: int, layout: int, path: int = PATH_AUTO) -> int:
@@ -235,12 +227,6 @@ class Workspace:
         return self.buf
 
 
-def _weight_kn(q: QuantizedTensor, layout: int):
-    if len(q.original_shape) != 2:
-        raise RuntimeError("matmul currently requires 2D tensors!")          # src/ops.cpp:380-382
-    return (q.original_shape[0], q.original_shape[1]) if layout == LAYOUT_KN else (q.original_shape[1], q.original_shape[0])
-
-
 def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: Optional[torch.Tensor] = None, *, layout: int = LAYOUT_KN,
                      path: int = PATH_AUTO, out: Optional[torch.Tensor] = None, workspace: Optional[Workspace] = None,
                      ldy: Optional[int] = None, workspace_limit: Optional[int] = None) -> torch.Tensor:
@@ -248,63 +234,14 @@ def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: Optional[torch.T
     layout=LAYOUT_KN is the reference's own convention (weight [K,N], y = x*W).  workspace_limit caps the scratch
     bytes offered to the library (the bf16 tensor-core path then dequantizes [N,K] weights tile by tile in shared
     memory instead of expanding them into the scratch first)."""
-    x = _f32_cuda(x)
-    if x.dim() != 2:
-        raise RuntimeError("matmul currently requires 2D tensors!")
-    K, N = _weight_kn(q, layout)
-    M = x.shape[0]
-    if x.shape[1] != K:
-        raise RuntimeError("Matrix inner dimensions must match for matmul!")   # src/ops.cpp:387-389
-    b = None if bias is None else _f32_cuda(bias).reshape(-1)
-    if b is not None and b.numel() != N:
-        raise RuntimeError("Incompatible shapes for broadcasting!")            # src/ops.cpp:60
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        ldy = N
-    elif ldy is None:
-        ldy = out.stride(0)
-    need = linear_workspace_bytes(q.bits, M, K, N, layout, path)
-    if workspace_limit is not None:
-        need = min(need, workspace_limit)
-    ws = None
-    if need:
-        ws = (workspace or Workspace(x.device)).get(need)
-    wsp, wsb = (_ptr(ws), ws.numel()) if ws is not None else (None, 0)
-    if workspace_limit is not None:
-        wsb = min(wsb, workspace_limit)
-    if q.bits == 4:
-        rc = lib.sgq_linear_int4(_ptr(x), M, K, N, _ptr(q.qdata), _ptr(q.scales), layout, q.group_size, _ptr(b), _ptr(out),
-                                 ldy, path, wsp, wsb, _stream())
-    else:
-        per_tensor = q.scheme == PER_TENSOR or q.scales.numel() == 1
-        rc = lib.sgq_linear_int8(_ptr(x), M, K, N, _ptr(q.qdata), _ptr(q.scales), layout,
-                                 PER_TENSOR if per_tensor else PER_ROW, _ptr(b), _ptr(out), ldy, path, wsp, wsb, _stream())
-    check(rc, "sgq_linear")
-    return out
+    return _native.quantized_matmul(x, q, bias, layout, path, out, workspace, ldy, workspace_limit)
 
 
 def quantized_matmul_backward_x(dy: torch.Tensor, q: QuantizedTensor, *, layout: int = LAYOUT_KN, path: int = PATH_AUTO,
                                 workspace: Optional[Workspace] = None) -> torch.Tensor:
     """Gradient with respect to x of quantized_matmul(x, q): what the reference's autograd computes through
     quantized_matmul_int8 / _int4 when x requires a gradient (src/ops.cpp:367-370, 451-453)."""
-    dy = _f32_cuda(dy)
-    K, N = _weight_kn(q, layout)
-    M = dy.shape[0]
-    if dy.dim() != 2 or dy.shape[1] != N:
-        raise RuntimeError("Matrix inner dimensions must match for matmul!")
-    dx = torch.empty((M, K), dtype=torch.float32, device=dy.device)
-    need = int(lib.sgq_linear_backward_x_workspace_bytes(q.bits, M, K, N, layout, path))
-    ws = (workspace or Workspace(dy.device)).get(need) if need else None
-    wsp, wsb = (_ptr(ws), ws.numel()) if ws is not None else (None, 0)
-    if q.bits == 4:
-        rc = lib.sgq_linear_int4_backward_x(_ptr(dy), M, K, N, _ptr(q.qdata), _ptr(q.scales), layout, q.group_size, _ptr(dx), K, path,
-                                            wsp, wsb, _stream())
-    else:
-        per_tensor = q.scheme == PER_TENSOR or q.scales.numel() == 1
-        rc = lib.sgq_linear_int8_backward_x(_ptr(dy), M, K, N, _ptr(q.qdata), _ptr(q.scales), layout,
-                                            PER_TENSOR if per_tensor else PER_ROW, _ptr(dx), K, path, wsp, wsb, _stream())
-    check(rc, "sgq_linear_backward_x")
-    return dx
+    return _native.backward_x(dy, q, layout, path, workspace)
 
 
 def quantize_activations_int8(x: torch.Tensor):
@@ -357,22 +294,7 @@ def quantized_matmul_int4(x, q_weight, bias=None, **kw):
 def linear_w8a8(x: torch.Tensor, q: QuantizedTensor, bias: Optional[torch.Tensor] = None, *, want_parts: bool = False):
     """Integer sub-path (no counterpart in the reference): per-row INT8 activations, exact int32
     accumulation on tcgen05 kind::i8.  Weight must be INT8 stored [N,K]."""
-    x = _f32_cuda(x)
-    N, K = q.original_shape
-    M = x.shape[0]
-    y = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    xq = sx = acc = None
-    if want_parts:
-        xq = torch.empty((M, K), dtype=torch.int8, device=x.device)
-        sx = torch.empty(M, dtype=torch.float32, device=x.device)
-        acc = torch.empty((M, N), dtype=torch.int32, device=x.device)
-    nb = int(lib.sgq_linear_w8a8_workspace_bytes(M, K, N))
-    ws = torch.empty(max(nb, 256), dtype=torch.uint8, device=x.device)
-    b = None if bias is None else _f32_cuda(bias).reshape(-1)
-    per_tensor = q.scheme == PER_TENSOR or q.scales.numel() == 1
-    check(lib.sgq_linear_w8a8(_ptr(x), M, K, N, _ptr(q.qdata), _ptr(q.scales), PER_TENSOR if per_tensor else PER_ROW, _ptr(b),
-                              _ptr(y), N, _ptr(xq), _ptr(sx), _ptr(acc), _ptr(ws), ws.numel(), _stream()), "sgq_linear_w8a8")
-    return (y, xq, sx, acc) if want_parts else y
+    return _native.linear_w8a8(x, q, bias, want_parts)
 
 
 def interleave_slices(gathered: torch.Tensor, world: int, M: int, n_local: int, out: Optional[torch.Tensor] = None):
@@ -404,7 +326,7 @@ class QuantizedLinear:
         return {"qdata": self.q_weight.qdata, "scales": self.q_weight.scales, "bias": self.bias}
 
     def forward(self, x: torch.Tensor, path: int = PATH_AUTO) -> torch.Tensor:
-        return quantized_matmul(x, self.q_weight, self.bias, layout=self.layout, path=path, workspace=self._ws)
+        return _native.quantized_matmul(x, self.q_weight, self.bias, self.layout, path, None, self._ws, None, None)
 
     __call__ = forward
 

@@ -20,6 +20,8 @@ OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(LIB_DIR, "libsgq.so")
 SOURCES = ["abi.cu", "quantize.cu", "linear_simt.cu", "gemv.cu", "gemm_tc.cu", "decoder_glue.cu", "peer.cu", "gemv_i8.cu", "linear_kn.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr"]
 
@@ -57,14 +59,33 @@ def build(force: bool = False, verbose: bool = False) -> str:
         # cudart is linked statically; the driver entry point for tensor maps is resolved at run time
         subprocess.check_call([NVCC, "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
                                "-Xcompiler", "-fPIC"])
+    build_binding(force)
     return LIB
+
+
+BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
+BINDING = os.path.join(LIB_DIR, "_sgq_torch.so")
+
+
+def build_binding(force: bool = False) -> str:
+    """The Python package's native calls (csrc/torch_binding.cpp), against the installed torch's headers."""
+    if force or _stale(BINDING, [BINDING_SRC, os.path.join(os.path.dirname(HERE), "include", "sgq.h")]):
+        import sysconfig
+
+        import torch
+        t = os.path.dirname(torch.__file__)
+        inc = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(CUDA_HOME, "include")]
+        subprocess.check_call([CXX, "-std=c++17", "-O2", "-fPIC", "-shared", "-Wall", "-fvisibility=hidden",
+                               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in inc], BINDING_SRC,
+                               "-o", BINDING, "-L", LIB_DIR, "-lsgq", "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch",
+                               "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
+    return BINDING
 
 
 HOST_DIR = os.path.join(HERE, "host")
 HOST_LIB = os.path.join(LIB_DIR, "libsgq_host.so")
 HOST_TEST = os.path.join(LIB_DIR, "sgq_host_test")
-CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 
 def build_host(force: bool = False) -> str:
