@@ -846,7 +846,7 @@ int launch_attn(const float* qkv, int64_t qkv_stride, int64_t batch, int n_heads
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = stream_overlap_enabled() ? 2 : 1;
+    cfg.numAttrs = 2;
     if (peers.n > 0) {
         SGQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, attn_decode_kernel<HD, true>, qkv, qkv_stride, n_heads, cos_t, sin_t, kc, vc, max_seq, pos0,
                                         out, out_stride, static_cast<int>(batch), L.mode, L.nmain, L.nlow, planes, peers));
@@ -892,14 +892,13 @@ int sgqd_add_rmsnorm(float* h, const float* delta, const float* gamma, float eps
     rc = check_device();
     if (rc != SGQ_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool ov = stream_overlap_enabled();
     const bool in_regs = (dim % 256) == 0 && dim <= 8192 && aligned(h, 16) && aligned(out, 16) && aligned(gamma, 16) &&
                          (!delta || aligned(delta, 16));
     if (in_regs) {
         uint8_t* pl = static_cast<uint8_t*>(prepared_out);
         const dim3 grid(static_cast<unsigned>(rows)), block(kNormThreads);
 #define SGQ_NORM_ROW(PREPV, CHV) \
-    SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_row_kernel<PREPV, CHV>, grid, block, 0, s, ov, h, delta, gamma, eps, dim, out, L.mode, L.nmain, L.nlow, pl))
+    SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_row_kernel<PREPV, CHV>, grid, block, 0, s, true, h, delta, gamma, eps, dim, out, L.mode, L.nmain, L.nlow, pl))
         if (dim <= 2048) { if (pl) SGQ_NORM_ROW(true, 1); else SGQ_NORM_ROW(false, 1); }
         else if (dim <= 4096) { if (pl) SGQ_NORM_ROW(true, 2); else SGQ_NORM_ROW(false, 2); }
         else { if (pl) SGQ_NORM_ROW(true, 4); else SGQ_NORM_ROW(false, 4); }
@@ -907,10 +906,10 @@ int sgqd_add_rmsnorm(float* h, const float* delta, const float* gamma, float eps
         return SGQ_OK;
     }
     if (prepared_out)
-        SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_kernel<true>, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, s, ov, h, delta,
+        SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_kernel<true>, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, s, true, h, delta,
                                    gamma, eps, dim, out, L.mode, L.nmain, L.nlow, static_cast<uint8_t*>(prepared_out)));
     else
-        SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_kernel<false>, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, s, ov, h, delta,
+        SGQ_CUDA_TRY(launch_kernel(add_rmsnorm_kernel<false>, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, s, true, h, delta,
                                    gamma, eps, dim, out, 0, 1, 1, static_cast<uint8_t*>(nullptr)));
     return SGQ_OK;
 }
@@ -926,7 +925,7 @@ int sgqd_rope_kv_store(float* qkv, int64_t batch, int64_t t_new, int64_t n_heads
     int rc = check_device();
     if (rc != SGQ_OK) return rc;
     SGQ_CUDA_TRY(launch_kernel(rope_kv_store_kernel, dim3(static_cast<unsigned>(batch * t_new)), dim3(256), 0,
-                               static_cast<cudaStream_t>(stream), stream_overlap_enabled(), qkv, static_cast<int>(t_new),
+                               static_cast<cudaStream_t>(stream), true, qkv, static_cast<int>(t_new),
                                static_cast<int>(n_heads), static_cast<int>(head_dim), cos_table, sin_table, pos0, k_cache, v_cache,
                                max_seq));
     return SGQ_OK;
@@ -1004,7 +1003,7 @@ int sgqd_silu_mul_allgather(const float* gate_up, int64_t rows, int64_t hidden, 
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
     SGQ_CUDA_TRY(launch_kernel(silu_mul_peers_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                               stream_overlap_enabled(), gate_up, rows, hidden, ld, peers));
+                               true, gate_up, rows, hidden, ld, peers));
     return SGQ_OK;
 }
 
@@ -1024,10 +1023,10 @@ int sgqd_attn_prefill(const float* qkv, int64_t qkv_stride, int64_t batch, int64
     const dim3 grid(static_cast<unsigned>(ceil_div(t_new, kPrefillQ)), static_cast<unsigned>(batch * n_heads));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (head_dim == 128)
-        SGQ_CUDA_TRY(launch_kernel(attn_prefill_kernel<128>, grid, dim3(256), 0, s, stream_overlap_enabled(), qkv, qkv_stride,
+        SGQ_CUDA_TRY(launch_kernel(attn_prefill_kernel<128>, grid, dim3(256), 0, s, true, qkv, qkv_stride,
                                    static_cast<int>(t_new), static_cast<int>(n_heads), k_cache, v_cache, max_seq, pos0, out, out_stride));
     else
-        SGQ_CUDA_TRY(launch_kernel(attn_prefill_kernel<64>, grid, dim3(256), 0, s, stream_overlap_enabled(), qkv, qkv_stride,
+        SGQ_CUDA_TRY(launch_kernel(attn_prefill_kernel<64>, grid, dim3(256), 0, s, true, qkv, qkv_stride,
                                    static_cast<int>(t_new), static_cast<int>(n_heads), k_cache, v_cache, max_seq, pos0, out, out_stride));
     return SGQ_OK;
 }
@@ -1046,7 +1045,7 @@ int sgqd_attn_prefill_bf16(const float* qkv, int64_t qkv_stride, int64_t batch, 
     int rc = check_device();
     if (rc != SGQ_OK) return rc;
     const dim3 grid(static_cast<unsigned>(ceil_div(t_new, kTcQ)), static_cast<unsigned>(batch * n_heads));
-    SGQ_CUDA_TRY(launch_kernel(attn_prefill_tc_kernel, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), stream_overlap_enabled(), qkv,
+    SGQ_CUDA_TRY(launch_kernel(attn_prefill_tc_kernel, grid, dim3(128), 0, static_cast<cudaStream_t>(stream), true, qkv,
                                qkv_stride, static_cast<int>(t_new), static_cast<int>(n_heads), k_cache, v_cache, max_seq, pos0, out,
                                out_stride));
     return SGQ_OK;
@@ -1060,7 +1059,7 @@ int sgqd_embedding(const float* table, int64_t vocab, int64_t dim, const int64_t
     if (rc != SGQ_OK) return rc;
     const int vec = ((dim & 3) == 0 && aligned(table, 16) && aligned(out, 16)) ? 1 : 0;
     SGQ_CUDA_TRY(launch_kernel(embedding_kernel, dim3(static_cast<unsigned>(rows)), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                               stream_overlap_enabled(), table, vocab, dim, ids, out, vec));
+                               true, table, vocab, dim, ids, out, vec));
     return SGQ_OK;
 }
 
@@ -1071,7 +1070,7 @@ int sgqd_argmax_rows(const float* x, int64_t rows, int64_t n, int64_t ld, int64_
     int rc = check_device();
     if (rc != SGQ_OK) return rc;
     SGQ_CUDA_TRY(launch_kernel(argmax_rows_kernel, dim3(static_cast<unsigned>(rows)), dim3(kArgmaxThreads), 0,
-                               static_cast<cudaStream_t>(stream), stream_overlap_enabled(), x, n, ld, out));
+                               static_cast<cudaStream_t>(stream), true, x, n, ld, out));
     return SGQ_OK;
 }
 
@@ -1090,20 +1089,20 @@ int sgqd_silu_mul(const float* gate_up, int64_t rows, int64_t hidden, float* out
     if (prepared_out && (hidden % 256) == 0 && hidden / 8 <= 65535LL * kSiluThreads) {
         SGQ_CUDA_TRY(launch_kernel(silu_mul_prepare_row_kernel,
                                    dim3(static_cast<unsigned>(rows), static_cast<unsigned>(ceil_div(hidden / 8, kSiluThreads))), dim3(kSiluThreads), 0, s,
-                                   stream_overlap_enabled(), gate_up, hidden, out, L.mode, L.nmain, L.nlow,
+                                   true, gate_up, hidden, out, L.mode, L.nmain, L.nlow,
                                    static_cast<uint8_t*>(prepared_out)));
         return SGQ_OK;
     }
     if (prepared_out) {
         SGQ_CUDA_TRY(launch_kernel(silu_mul_prepare_kernel, dim3(static_cast<unsigned>(rows)), dim3(kNormThreads), 0, s,
-                                   stream_overlap_enabled(), gate_up, hidden, out, L.mode, L.nmain, L.nlow,
+                                   true, gate_up, hidden, out, L.mode, L.nmain, L.nlow,
                                    static_cast<uint8_t*>(prepared_out)));
         return SGQ_OK;
     }
     int64_t blocks = ceil_div(rows * hidden, 256);
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
-    SGQ_CUDA_TRY(launch_kernel(silu_mul_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, stream_overlap_enabled(), gate_up,
+    SGQ_CUDA_TRY(launch_kernel(silu_mul_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, true, gate_up,
                                rows, hidden, out));
     return SGQ_OK;
 }

@@ -849,8 +849,8 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
             // while the rest is still being expanded.
             const int64_t wsteps = a.N * a.K / 8;
             const int64_t most = wsteps > chunks ? wsteps : chunks;
-            // (without overlapped launches the GEMM starts behind the whole expansion anyway: then the grid fills the
-            // machine and the weight is one slice)
+            // (the expansion itself is an ordinary launch: when it starts, everything older is complete, so the GEMM that
+            // starts beside it finds the outputs free whatever sgq_set_stream_overlap says)
             // Beside the GEMM only while the register budget of an SM quarter holds: 2 GEMM warps of at most 160
             // registers a thread next to 4 expansion warps of 48 (16384 in all); a compiler that needs more for
             // the GEMM gets the serial form instead of a silent loss of the overlap.
@@ -858,7 +858,7 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
                 cudaFuncAttributes fa{};
                 return cudaFuncGetAttributes(&fa, linear_tc_kernel<kBF16Plain>) == cudaSuccess && fa.numRegs <= 160;
             }();
-            const bool beside = stream_overlap_enabled() && fits && a.peers.n == 0;
+            const bool beside = fits && a.peers.n == 0;
             const int64_t wave = static_cast<int64_t>(sm_count()) * (beside ? kExpandCtasPerSm : 16);
             const int egrid = static_cast<int>(ceil_div(most, 1024) < wave ? ceil_div(most, 1024) : wave);
             const int64_t kblocks = a.K / 64;
@@ -872,9 +872,9 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
                                                           round_up(static_cast<size_t>(a.N) * static_cast<size_t>(a.K) * 2, 256));
             SGQ_CUDA_TRY(cudaMemsetAsync(ready, 0, kReadyBytes, a.stream));
             const uint32_t N32 = static_cast<uint32_t>(a.N), K32 = static_cast<uint32_t>(a.K), M32 = static_cast<uint32_t>(a.M);
-            if (stream_overlap_enabled())     // the GEMM's CTA can only join an SM that runs under the same memory split
-                prefer_max_shared(a.bits == 4 ? reinterpret_cast<const void*>(expand_nk_ordered_kernel<4>)
-                                              : reinterpret_cast<const void*>(expand_nk_ordered_kernel<8>));
+            // the GEMM's CTA can only join an SM that runs under the same memory split
+            prefer_max_shared(a.bits == 4 ? reinterpret_cast<const void*>(expand_nk_ordered_kernel<4>)
+                                          : reinterpret_cast<const void*>(expand_nk_ordered_kernel<8>));
             if (a.bits == 4)
                 expand_nk_ordered_kernel<4><<<egrid, 256, 0, a.stream>>>(static_cast<const uint8_t*>(a.wq), a.scales,
                                                                         static_cast<uint32_t>(a.group), N32, K32, parts,
@@ -896,7 +896,7 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
         if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, wt, static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.N),
                                 static_cast<uint64_t>(a.K) * 2, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B))
             return SGQ_ERR_CUDA;
-        return launch_tc<kBF16Plain>(ma, mb, p, a.stream, p.ready != nullptr && stream_overlap_enabled());
+        return launch_tc<kBF16Plain>(ma, mb, p, a.stream, p.ready != nullptr);
     }
     if (a.bits == 8) {
         if (!make_tensor_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.wq, static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.N),

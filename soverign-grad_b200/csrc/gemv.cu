@@ -135,9 +135,14 @@ constexpr int kPrepThreads = 128;
 __global__ void __launch_bounds__(kPrepThreads) gemv_prepare_x_kernel(const float* __restrict__ x, int64_t K, int mode, int nmain,
                                                                      int nlow, uint8_t* __restrict__ planes,
                                                                      const unsigned long long* wait_slots, int wait_world,
-                                                                     const unsigned long long* wait_epoch, unsigned int wait_budget) {
-    pdl_launch_dependents();
+                                                                     const unsigned long long* wait_epoch, unsigned int wait_budget,
+                                                                     int trigger_first) {
+    // The decode kernel behind this one requests its first weights as soon as it starts.  Triggered behind the wait, it
+    // starts when everything in front of this kernel is complete, so those loads need no rule of the caller's; with
+    // overlapped launches (weights are no recent output, sgq_set_stream_overlap) it may start earlier still.
+    if (trigger_first) pdl_launch_dependents();
     pdl_wait();                                        // x comes from the kernel before this one
+    if (!trigger_first) pdl_launch_dependents();
     // Deferred exchange between GPUs: x may hold slices that other GPUs store, so this kernel waits as the decode
     // kernel itself does in its prologue (every rank has finished the exchanges this GPU has finished).
     if (wait_slots != nullptr && !peer_wait_epoch(wait_slots, wait_world, wait_epoch, threadIdx.x & 31, wait_budget)) {
@@ -696,12 +701,15 @@ int launch_variant(const LinearArgs& a, const Plan& p, const CUtensorMap& map_w,
     const bool overlap = stream_overlap_enabled();
     if (p.pre && !planes_ready) {
         const bool wait = a.peers.n > 0 && a.peers.deferred && a.peers.sig[0] != nullptr;
-        SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(a.M), static_cast<unsigned>(ceil_div(a.K / 8, kPrepThreads))), dim3(kPrepThreads), 0, a.stream, overlap,
+        SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(a.M), static_cast<unsigned>(ceil_div(a.K / 8, kPrepThreads))), dim3(kPrepThreads), 0, a.stream, true,
                                    a.x, a.K, p.L.mode, p.L.nmain, p.L.nlow, static_cast<uint8_t*>(a.workspace),
-                                   wait ? a.peers.sig[a.peers.rank] : nullptr, a.peers.n, a.peers.state, a.peers.poll_budget));
+                                   wait ? a.peers.sig[a.peers.rank] : nullptr, a.peers.n, a.peers.state, a.peers.poll_budget, overlap ? 1 : 0));
     }
-    const int flags = (overlap ? kFlagEarlyWeights : 0) | (p.pre ? kFlagPrepared : 0);
-    SGQ_CUDA_TRY(launch_kernel(kernel, dim3(static_cast<unsigned>(grid)), dim3((NWARPS + 2) * 32), p.smem, a.stream, overlap, map_w,
+    // Early weights: with overlapped launches always; otherwise behind the conversion launch, which lets this kernel
+    // start only when everything in front of the call is complete.
+    const bool early = overlap || (p.pre && !planes_ready);
+    const int flags = (early ? kFlagEarlyWeights : 0) | (p.pre ? kFlagPrepared : 0);
+    SGQ_CUDA_TRY(launch_kernel(kernel, dim3(static_cast<unsigned>(grid)), dim3((NWARPS + 2) * 32), p.smem, a.stream, true, map_w,
                                map_s, a.x, planes, a.bias, a.y, static_cast<int>(a.M), a.K, a.N, a.ldy, p.nstages, p.nphases, flags,
                                a.peers));
     return SGQ_OK;
@@ -755,8 +763,8 @@ size_t gemv_prepared_bytes(int64_t M, int64_t K) {
 int launch_prepare_x(const float* x, int64_t M, int64_t K, void* prepared, cudaStream_t s) {
     const PreparedLayout L = prepared_layout(M, K);
     SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(M), static_cast<unsigned>(ceil_div(K / 8, kPrepThreads))), dim3(kPrepThreads), 0, s,
-                               stream_overlap_enabled(), x, K, L.mode, L.nmain, L.nlow, static_cast<uint8_t*>(prepared),
-                               static_cast<const unsigned long long*>(nullptr), 0, static_cast<const unsigned long long*>(nullptr), 0u));
+                               true, x, K, L.mode, L.nmain, L.nlow, static_cast<uint8_t*>(prepared),
+                               static_cast<const unsigned long long*>(nullptr), 0, static_cast<const unsigned long long*>(nullptr), 0u, 1));
     return SGQ_OK;
 }
 

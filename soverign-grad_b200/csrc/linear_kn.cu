@@ -161,14 +161,13 @@ KnPlan kn_plan(int64_t M, int64_t K, int64_t N) {
 
 template <int BITS, int MB>
 int launch_pass(const LinearArgs& a, const KnPlan& p, int scale_mode, const float* x, float* y, int rows, float* part) {
-    const bool overlap = stream_overlap_enabled();
     SGQ_CUDA_TRY(launch_kernel(kn_partial_kernel<BITS, MB>, dim3(static_cast<unsigned>(p.nblocks), static_cast<unsigned>(p.slices)),
-                               dim3(kThreads), 0, a.stream, overlap, x, a.K, a.N, static_cast<const uint8_t*>(a.wq), a.scales,
+                               dim3(kThreads), 0, a.stream, true, x, a.K, a.N, static_cast<const uint8_t*>(a.wq), a.scales,
                                scale_mode, a.group, p.slice_k, part));
     int64_t blocks = ceil_div(static_cast<int64_t>(rows) * a.N, 256);
     const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
     if (blocks > cap) blocks = cap;
-    SGQ_CUDA_TRY(launch_kernel(kn_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, a.stream, overlap,
+    SGQ_CUDA_TRY(launch_kernel(kn_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, a.stream, true,
                                static_cast<const float*>(part), p.slices, MB, a.N, a.bias, y, a.ldy));
     (void)rows;
     return SGQ_OK;

@@ -93,7 +93,7 @@ int sgq_peer_scatter(const float* src, int64_t M, int64_t n_local, float* const*
     if (blocks < 1) blocks = 1;
     // 128-bit stores when every row on both sides is 16-byte aligned
     SGQ_CUDA_TRY(launch_kernel(peer_scatter_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                               stream_overlap_enabled(), src, M, n_local, peers, ldy, vec ? 1 : 0));
+                               true, src, M, n_local, peers, ldy, vec ? 1 : 0));
     return SGQ_OK;
 }
 
@@ -107,7 +107,7 @@ int sgq_peer_barrier(void* const* signals, int rank, int world, void* local_epoc
     }
     int rc = check_device();
     if (rc != SGQ_OK) return rc;
-    SGQ_CUDA_TRY(launch_kernel(peer_barrier_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(stream), stream_overlap_enabled(),
+    SGQ_CUDA_TRY(launch_kernel(peer_barrier_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(stream), true,
                                sig, rank, world, static_cast<unsigned long long*>(local_epoch), peer_wait_budget()));
     return SGQ_OK;
 }

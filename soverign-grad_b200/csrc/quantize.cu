@@ -384,15 +384,14 @@ int launch_quantize_int8(const float* x, int64_t rows, int64_t cols, int scheme,
                          cudaStream_t s) {
     const int64_t n = rows * cols;
     if (scheme == SGQ_PER_TENSOR) {
-        const bool ov = stream_overlap_enabled();
-        SGQ_CUDA_TRY(launch_kernel(set_f32_kernel, dim3(1), dim3(1), 0, s, ov, scales, 1e-8f));
+        SGQ_CUDA_TRY(launch_kernel(set_f32_kernel, dim3(1), dim3(1), 0, s, true, scales, 1e-8f));
         if (n > 0) {
             const int grid = grid_for(n, kThreads * 16, 8);
-            SGQ_CUDA_TRY(launch_kernel(tensor_absmax_kernel, dim3(grid), dim3(kThreads), 0, s, ov, x, n, scales));
-            SGQ_CUDA_TRY(launch_kernel(quantize_int8_tensor_kernel, dim3(grid), dim3(kThreads), 0, s, ov, x, n,
+            SGQ_CUDA_TRY(launch_kernel(tensor_absmax_kernel, dim3(grid), dim3(kThreads), 0, s, true, x, n, scales));
+            SGQ_CUDA_TRY(launch_kernel(quantize_int8_tensor_kernel, dim3(grid), dim3(kThreads), 0, s, true, x, n,
                                        static_cast<const float*>(scales), codes));
         }
-        SGQ_CUDA_TRY(launch_kernel(scale_from_absmax_pdl_kernel, dim3(1), dim3(kThreads), 0, s, ov, scales, static_cast<int64_t>(1), 127.0f));
+        SGQ_CUDA_TRY(launch_kernel(scale_from_absmax_pdl_kernel, dim3(1), dim3(kThreads), 0, s, true, scales, static_cast<int64_t>(1), 127.0f));
         return SGQ_OK;
     }
     if (rows == 0) return SGQ_OK;
