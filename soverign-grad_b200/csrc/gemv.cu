@@ -202,7 +202,7 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     uint64_t* xfull = pempty + kMaxSlots;      // the activation planes of a phase have landed
     uint64_t* xempty = xfull + 1;              // every consumer warp is done with the planes of a phase
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int64_t ntiles = (N + kRows - 1) / kRows;
     const int ring_slots = nstages / kGroups;          // stage slots per warp group (nstages >= kGroups)
     // Split form (no CTA has more than one tile, so one warp group would idle): the stages of the tile alternate
@@ -238,7 +238,7 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == NWARPS) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             // Weights and scales are parameters, not the output of the kernel before this one: with
             // early weights the first ring of stages is requested before the dependency wait, so the
             // weight stream overlaps the tail of that kernel.  The activation planes are its output

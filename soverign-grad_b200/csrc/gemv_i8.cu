@@ -192,7 +192,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     uint64_t* empty = full + kMaxStages;
     constexpr int kPStride = 128 * NM + 4;          // floats per warp in a partial-sum slot
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     // this CTA's tiles: a contiguous range, sizes differing by at most one (blocks of RT whole tiles per CTA would leave
     // up to a quarter of the machine idle in the last round)
     const int64_t ntiles = (N + kRows - 1) / kRows;
@@ -219,7 +219,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == kWarps) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             // steps past K/128 are out of range in the third dimension of a box: zero-filled, still counted
             auto weights = [&](uint32_t st, int b, int c0) {
                 const int32_t t0 = static_cast<int32_t>(tile0) + b * RT;
