@@ -15,6 +15,7 @@ cudaError_t read_status_gemv(uint32_t* v, bool clear);
 cudaError_t read_status_gemm(uint32_t* v, bool clear);
 cudaError_t read_status_peer(uint32_t* v, bool clear);
 cudaError_t read_status_gemv_i8(uint32_t* v, bool clear);
+cudaError_t read_status_kn(uint32_t* v, bool clear);
 
 namespace {
 thread_local char g_error[512] = "";
@@ -254,12 +255,13 @@ unsigned int sgq_set_peer_wait_budget(unsigned int polls) {
 }
 
 int sgq_device_status(unsigned int* word, int clear) {
-    uint32_t a = 0, b = 0, c = 0, d = 0;
-    SGQ_CUDA_TRY(read_status_gemv(&a, clear != 0));
-    SGQ_CUDA_TRY(read_status_gemm(&b, clear != 0));
-    SGQ_CUDA_TRY(read_status_peer(&c, clear != 0));
-    SGQ_CUDA_TRY(read_status_gemv_i8(&d, clear != 0));
-    const uint32_t v = a ? a : (b ? b : (c ? c : d));
+    cudaError_t (*const readers[])(uint32_t*, bool) = {read_status_gemv, read_status_gemm, read_status_peer, read_status_gemv_i8, read_status_kn};
+    uint32_t v = 0;
+    for (auto read : readers) {
+        uint32_t w = 0;
+        SGQ_CUDA_TRY(read(&w, clear != 0));
+        if (v == 0) v = w;
+    }
     if (word) *word = v;
     if (v != 0) {
         set_error("device status word 0x%08x (code %u, detail %u)", v, v >> 24, v & 0xFFFFFFu);
