@@ -1,0 +1,50 @@
+"""The CTA-pair GEMM (csrc/gemm_tc.cu) at the edges of its tiles: rows around the 128 of a CTA and the 256 of a pair, columns
+that end inside a tile, inside a half and inside a 64-column block, one k-block and more than the ring holds, several tiles
+per pair; both orders of the weight.  The oracle is a float64 product of the operands as the path rounds them."""
+import numpy as np
+import pytest
+
+import cases
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sgq():
+    from __graft_entry__ import load_package
+    return load_package()
+
+
+SHAPES = [(1, 64, 32), (64, 64, 96), (127, 128, 160), (128, 192, 416), (129, 512, 288), (255, 576, 1056), (256, 1024, 4064),
+          (257, 64, 22016), (300, 448, 2080), (600, 640, 9632), (2500, 256, 2592)]
+
+
+def check(y, x, w, K):
+    want = x.double() @ w.double()
+    mag = x.double().abs() @ w.double().abs()
+    # exact products, fp32 sums of K of them (one rounding of at most 2^-23 of the running magnitude each) and the epilogue's two
+    assert bool(((y.double() - want).abs() <= mag * (K + 4) * 2.0 ** -23 + 1e-12).all())
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+def test_pair_gemm_edges(sgq, M, K, N):
+    gen = torch.Generator(device="cuda").manual_seed(M * 7 + K * 3 + N)
+    x = torch.randn(M, K, device="cuda", generator=gen)
+    b = torch.randn(N, device="cuda", generator=gen)
+    xb = x.bfloat16()
+    ws = sgq.Workspace(torch.device("cuda"))
+    for layout in (cases.LAYOUT_NK, cases.LAYOUT_KN):
+        n = N - 3 if layout == cases.LAYOUT_NK else N               # rows of 4n bytes: also the epilogue without 128-bit stores
+        w = torch.randn((n, K) if layout == cases.LAYOUT_NK else (K, n), device="cuda", generator=gen) * 0.05
+        for q, deq in ((sgq.quantize_int4(w, 32), sgq.dequantize_int4),
+                       (sgq.quantize_int8(w, cases.PER_ROW), sgq.dequantize_int8),
+                       (sgq.quantize_int8(w, cases.PER_TENSOR), sgq.dequantize_int8)):
+            real = deq(q)
+            # the scales of INT8 codes stored [N,K] multiply the sums in fp32; else code * scale is rounded to bf16
+            wf = real if q.qdata.dtype == torch.int8 and layout == cases.LAYOUT_NK else real.bfloat16().float()
+            wf = wf.t() if layout == cases.LAYOUT_NK else wf
+            for bias in (None, b[:n]):
+                y = sgq.quantized_matmul(x, q, bias, layout=layout, path=sgq.PATH_TC_BF16, workspace=ws)
+                assert sgq.device_status() == 0
+                check(y if bias is None else y.double() - bias.double(), xb, wf, K + (0 if bias is None else 4096))
