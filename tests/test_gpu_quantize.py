@@ -127,3 +127,16 @@ def test_code_views_round_trip(sgq):
         sgq.check(fn(out.data_ptr(), 1001, back.data_ptr(), None))
         torch.cuda.synchronize()
         assert np.array_equal(host(back), c)
+
+
+@pytest.mark.parametrize("rows,cols,group", [(1, 3, 32), (3, 4, 4), (5, 36, 12), (7, 1001, 32), (33, 4100, 64), (64, 4096, 128), (2, 2051, 6)])
+def test_dequantize_vector_and_tail(sgq, port, rows, cols, group):
+    """Sizes with and without whole quads per row and group, tails of one to three codes: the products are exact, so bits are."""
+    w = cases.weight_with_outliers(rows * cols, (rows, cols))
+    for scheme in (cases.PER_TENSOR, cases.PER_ROW):
+        codes, scales = port.quantize_int8(w, scheme)
+        q = sgq.quantize_int8(torch.from_numpy(w).cuda(), scheme)
+        assert np.array_equal(sgq.dequantize_int8(q).cpu().numpy(), port.dequantize_int8(codes, scales, scheme).reshape(rows, cols))
+    packed, scales = port.quantize_int4(w, group)
+    q = sgq.quantize_int4(torch.from_numpy(w).cuda(), group)
+    assert np.array_equal(sgq.dequantize_int4(q).cpu().numpy(), port.dequantize_int4(packed, scales, (rows, cols), group))
