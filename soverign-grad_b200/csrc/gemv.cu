@@ -511,6 +511,26 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                             uint32_t wv[BG / 2][4];                      // [pair of groups]{rows 0-7, rows 8-15} x 2
 #pragma unroll
                             for (int pq = 0; pq < BG / 2; ++pq) ldmatrix_x4(wv[pq], wbox + lm_off[(hb * BG) / 2 + pq]);
+                            // Low digits: only where a row of the set flagged the group (one value dominating it: rare in a
+                            // normalised row, common behind a gate).  They lie in global memory, so the fragments of all
+                            // flagged groups are requested together, before the main MMAs; fetched one by one where they
+                            // are used they cost an L2 round trip per group.
+                            uint2 lowq[BG][NL > 0 ? NL : 1];
+                            float2 lowsc[BG][NL > 0 ? NL : 1];
+                            uint32_t flagged = 0;                        // bit i * NL + l, the same in every lane of the warp
+#pragma unroll
+                            for (int i = 0; i < BG; ++i) {
+#pragma unroll
+                                for (int l = 0; l < NL; ++l) {
+                                    const uint2 fl = *reinterpret_cast<const uint2*>(fg + (hb * BG + i) * 16 + l * 8);
+                                    if ((fl.x | fl.y) != 0u) {
+                                        const size_t grp = static_cast<size_t>(step) * 8 + hb * BG + i;       // group within the phase
+                                        flagged |= 1u << (i * NL + l);
+                                        lowq[i][l] = *reinterpret_cast<const uint2*>(lowd + plane_offset(grp, NL, l, lane));
+                                        lowsc[i][l] = *reinterpret_cast<const float2*>(lows + ((grp * 4 + t) * NL + l) * 2);
+                                    }
+                                }
+                            }
                             // The main-set MMAs of these groups are issued before any of their results is used, so
                             // that the tensor-pipe latency of one group is covered by the issue of the others.
                             int d[BG][NM][4];
@@ -542,7 +562,7 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                             }
 #pragma unroll
                             for (int i = 0; i < BG; ++i) {
-                                const int gi = hb * BG + i, gq = gi & 3;
+                                const int gq = (hb * BG + i) & 3;
                                 const float s_lo = gq == 0 ? sc_lo.x : gq == 1 ? sc_lo.y : gq == 2 ? sc_lo.z : sc_lo.w;
                                 const float s_hi = gq == 0 ? sc_hi.x : gq == 1 ? sc_hi.y : gq == 2 ? sc_hi.z : sc_hi.w;
 #pragma unroll
@@ -560,14 +580,11 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                                         total[s2][3] = __fmaf_rn(e_hi, __fsub_rn(__int_as_float(d[i][s2][3]), kMagicF), total[s2][3]);
                                     }
                                 }
-                                // low digits: only where a row of the set flagged this group (rare: one value dominating its group)
 #pragma unroll
                                 for (int l = 0; l < NL; ++l) {
-                                    const uint2 fl = *reinterpret_cast<const uint2*>(fg + gi * 16 + l * 8);
-                                    if ((fl.x | fl.y) != 0u) {           // the same for every lane of the warp
-                                        const size_t grp = static_cast<size_t>(step) * 8 + gi;       // group within the phase
-                                        const uint2 q = *reinterpret_cast<const uint2*>(lowd + plane_offset(grp, NL, l, lane));
-                                        const float2 sl = *reinterpret_cast<const float2*>(lows + ((grp * 4 + t) * NL + l) * 2);
+                                    if ((flagged >> (i * NL + l)) & 1u) {
+                                        const uint2 q = lowq[i][l];
+                                        const float2 sl = lowsc[i][l];
                                         int dl[4];
                                         mma_s8s8_16832_magic(dl, av[i], q.x, q.y);
                                         total[NM + l][0] = __fmaf_rn(__fmul_rn(s_lo, sl.x), __fsub_rn(__int_as_float(dl[0]), kMagicF), total[NM + l][0]);
