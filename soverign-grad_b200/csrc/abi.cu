@@ -179,7 +179,9 @@ int run_linear(LinearArgs a, int path) {
         LinearArgs blk = a;
         blk.M = kDecodeRows;
         if (decode_path_ready(blk)) {
-            for (int64_t m0 = 0; m0 < a.M; m0 += kDecodeRows) {
+            int64_t m0 = 0;
+            if (a.bits == 4 && a.layout == SGQ_LAYOUT_NK && a.group == 32 && (rc = launch_linear_gemv_blocks(a, &m0)) != SGQ_OK) return rc;
+            for (; m0 < a.M; m0 += kDecodeRows) {
                 LinearArgs sub = a;
                 sub.M = a.M - m0 < kDecodeRows ? a.M - m0 : kDecodeRows;
                 sub.x = a.x + m0 * a.K;
@@ -343,11 +345,17 @@ size_t sgq_linear_workspace_bytes(int bits, int64_t M, int64_t K, int64_t N, int
         case SGQ_PATH_TC_BF16: return tc_bf16_workspace_bytes(bits, M, K, N, layout);
         case SGQ_PATH_TC_I8: return tc_i8_workspace_bytes(M, K, N);
         default: {  // AUTO: enough for whichever path AUTO may take
-            if (M > 16 && M < 64) M = 16;       // runs as blocks of 16 rows that share the scratch
+            size_t blocks = 0;
+            if (M > kDecodeRows && M < kTensorCoreRows) {
+                // runs as blocks of 16 rows that share the scratch, or on planes that are all converted in front
+                if (bits == 4 && layout == SGQ_LAYOUT_NK) blocks = gemv_blocks_workspace_bytes(M, K);
+                M = kDecodeRows;
+            }
             size_t a = layout == SGQ_LAYOUT_KN ? kn_decode_workspace_bytes(bits, M, K, N)
                                                : (bits == 8 ? gemv_i8_workspace_bytes(M, K) : gemv_workspace_bytes(bits, M, K, N, layout));
-            size_t b = M >= 64 ? tc_bf16_workspace_bytes(bits, M, K, N, layout) : 0;
-            return a > b ? a : b;
+            size_t b = M >= kTensorCoreRows ? tc_bf16_workspace_bytes(bits, M, K, N, layout) : 0;
+            a = a > b ? a : b;
+            return a > blocks ? a : blocks;
         }
     }
 }

@@ -130,13 +130,14 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_addr
 }
 
 // Activation planes converted once into global scratch, in the prepared layout.  grid (rows, ceil(K / 1024)):
-// a CTA converts 1024 consecutive k of one row, so that even a few rows spread over many SMs.
+// a CTA converts 1024 consecutive k of one row, so that even a few rows spread over many SMs.  Every block_rows rows form a
+// prepared buffer of their own, block_bytes after the one before (a batch that several decode launches take).
 constexpr int kPrepThreads = 128;
 __global__ void __launch_bounds__(kPrepThreads) gemv_prepare_x_kernel(const float* __restrict__ x, int64_t K, int mode, int nmain,
                                                                      int nlow, uint8_t* __restrict__ planes,
                                                                      const unsigned long long* wait_slots, int wait_world,
                                                                      const unsigned long long* wait_epoch, unsigned int wait_budget,
-                                                                     int trigger_first) {
+                                                                     int trigger_first, int block_rows, size_t block_bytes) {
     // The decode kernel behind this one requests its first weights as soon as it starts.  Triggered behind the wait, it
     // starts when everything in front of this kernel is complete, so those loads need no rule of the caller's; with
     // overlapped launches (weights are no recent output, sgq_set_stream_overlap) it may start earlier still.
@@ -148,10 +149,10 @@ __global__ void __launch_bounds__(kPrepThreads) gemv_prepare_x_kernel(const floa
     if (wait_slots != nullptr && !peer_wait_epoch(wait_slots, wait_world, wait_epoch, threadIdx.x & 31, wait_budget)) {
         if ((threadIdx.x & 31) == 0) report(kDevErrPeerWait, 0x30000u);
     }
-    const int m = blockIdx.x, M = gridDim.x;
+    const int blk = static_cast<int>(blockIdx.x) / block_rows, m = static_cast<int>(blockIdx.x) - blk * block_rows, M = block_rows;
     const int chunks = static_cast<int>(K / 8);
-    const PreparedParts pp = prepared_parts(planes, static_cast<size_t>(K / 32), nmain, nlow);
-    const float4* xr = reinterpret_cast<const float4*>(x + static_cast<int64_t>(m) * K);
+    const PreparedParts pp = prepared_parts(planes + static_cast<size_t>(blk) * block_bytes, static_cast<size_t>(K / 32), nmain, nlow);
+    const float4* xr = reinterpret_cast<const float4*>(x + static_cast<int64_t>(blockIdx.x) * K);
     const int c = blockIdx.y * kPrepThreads + threadIdx.x;
     if (c < chunks) {                                  // chunks % 32 == 0: whole warps
         const float4 a = __ldg(xr + 2 * c), b = __ldg(xr + 2 * c + 1);
@@ -720,11 +721,12 @@ int launch_variant(const LinearArgs& a, const Plan& p, const CUtensorMap& map_w,
         const bool wait = a.peers.n > 0 && a.peers.deferred && a.peers.sig[0] != nullptr;
         SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(a.M), static_cast<unsigned>(ceil_div(a.K / 8, kPrepThreads))), dim3(kPrepThreads), 0, a.stream, true,
                                    a.x, a.K, p.L.mode, p.L.nmain, p.L.nlow, static_cast<uint8_t*>(a.workspace),
-                                   wait ? a.peers.sig[a.peers.rank] : nullptr, a.peers.n, a.peers.state, a.peers.poll_budget, overlap ? 1 : 0));
+                                   wait ? a.peers.sig[a.peers.rank] : nullptr, a.peers.n, a.peers.state, a.peers.poll_budget, overlap ? 1 : 0,
+                                   static_cast<int>(a.M), static_cast<size_t>(0)));
     }
     // Early weights: with overlapped launches always; otherwise behind the conversion launch, which lets this kernel
-    // start only when everything in front of the call is complete.
-    const bool early = overlap || (p.pre && !planes_ready);
+    // start only when everything in front of the call is complete (that of its whole batch: weights_settled).
+    const bool early = overlap || (p.pre && !planes_ready) || a.weights_settled;
     const int flags = (early ? kFlagEarlyWeights : 0) | (p.pre ? kFlagPrepared : 0);
     SGQ_CUDA_TRY(launch_kernel(kernel, dim3(static_cast<unsigned>(grid)), dim3((NWARPS + 2) * 32), p.smem, a.stream, true, map_w,
                                map_s, a.x, planes, a.bias, a.y, static_cast<int>(a.M), a.K, a.N, a.ldy, p.nstages, p.nphases, flags,
@@ -771,6 +773,56 @@ int launch_linear_gemv(const LinearArgs& a) { return launch_gemv_impl(a, false);
 // a.workspace holds activations already converted to the prepared format (a.x is not read).
 int launch_linear_gemv_prepared(const LinearArgs& a) { return launch_gemv_impl(a, true); }
 
+// Batches of 17 rows and more: how many rows from the first on go in equal blocks whose planes one conversion launch makes,
+// and the rows of a block.  These are the launches that blocks of 16 rows would split into anyway; 0: fewer than two such.
+int64_t gemv_block_rows(int64_t M, int64_t K, int64_t* rows) {
+    if (M <= kMaxM || !shape_ok(kMaxM, K, 1)) return 0;
+    Plan p;
+    const int64_t r = rows_per_launch(kMaxM, K, true);
+    if (r < 3 || kMaxM % r != 0 || !make_plan(r, K, true, &p) || !p.pre) return 0;
+    int64_t take = M / kMaxM * kMaxM;
+    if (M - take == r) take = M;
+    *rows = r;
+    return take >= 2 * r ? take : 0;
+}
+
+size_t gemv_blocks_workspace_bytes(int64_t M, int64_t K) {
+    int64_t rows = 0;
+    const int64_t take = gemv_block_rows(M, K, &rows);
+    return take ? static_cast<size_t>(take / rows) * gemv_prepared_bytes(rows, K) : 0;
+}
+
+// The first *taken rows of a batch of 17 and more: one conversion launch, then a decode launch per block.  Converting every
+// block in front of its own decode launch put 3 us between two of them (40 rows, W[4096,4096], five blocks: 47.0 us, now 40.3).
+int launch_linear_gemv_blocks(const LinearArgs& a, int64_t* taken) {
+    *taken = 0;
+    int64_t rows = 0;
+    const int64_t take = gemv_block_rows(a.M, a.K, &rows);
+    const size_t need = gemv_blocks_workspace_bytes(a.M, a.K);
+    if (take == 0 || a.peers.n != 0 || !a.workspace || !aligned(a.workspace, 256) || a.workspace_bytes < need) return SGQ_OK;
+    LinearArgs sub = a;
+    sub.M = rows;
+    if (!gemv_supported(sub) || stream_overlap_compact()) return SGQ_OK;
+    const PreparedLayout L = prepared_layout(rows, a.K);
+    const size_t bytes = gemv_prepared_bytes(rows, a.K);
+    uint8_t* planes = static_cast<uint8_t*>(a.workspace);
+    SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(take), static_cast<unsigned>(ceil_div(a.K / 8, kPrepThreads))),
+                               dim3(kPrepThreads), 0, a.stream, true, a.x, a.K, L.mode, L.nmain, L.nlow, planes,
+                               static_cast<const unsigned long long*>(nullptr), 0, static_cast<const unsigned long long*>(nullptr), 0u,
+                               stream_overlap_enabled() ? 1 : 0, static_cast<int>(rows), bytes));
+    sub.weights_settled = 1;
+    sub.workspace_bytes = bytes;
+    for (int64_t m0 = 0; m0 < take; m0 += rows) {
+        sub.workspace = planes + static_cast<size_t>(m0 / rows) * bytes;
+        sub.x = a.x + m0 * a.K;
+        sub.y = a.y + m0 * a.ldy;
+        const int rc = launch_linear_gemv_prepared(sub);
+        if (rc != SGQ_OK) return rc;
+    }
+    *taken = take;
+    return SGQ_OK;
+}
+
 size_t gemv_prepared_bytes(int64_t M, int64_t K) {
     Plan p;
     if (!shape_ok(M, K, 1) || !make_plan(M, K, true, &p)) return 0;
@@ -781,7 +833,8 @@ int launch_prepare_x(const float* x, int64_t M, int64_t K, void* prepared, cudaS
     const PreparedLayout L = prepared_layout(M, K);
     SGQ_CUDA_TRY(launch_kernel(gemv_prepare_x_kernel, dim3(static_cast<unsigned>(M), static_cast<unsigned>(ceil_div(K / 8, kPrepThreads))), dim3(kPrepThreads), 0, s,
                                true, x, K, L.mode, L.nmain, L.nlow, static_cast<uint8_t*>(prepared),
-                               static_cast<const unsigned long long*>(nullptr), 0, static_cast<const unsigned long long*>(nullptr), 0u, 1));
+                               static_cast<const unsigned long long*>(nullptr), 0, static_cast<const unsigned long long*>(nullptr), 0u, 1,
+                               static_cast<int>(M), static_cast<size_t>(0)));
     return SGQ_OK;
 }
 

@@ -198,6 +198,7 @@ struct LinearArgs {
     size_t workspace_bytes;
     cudaStream_t stream;
     PeerOut peers;        // decode kernel only
+    int weights_settled;  // decode kernel only: whoever wrote the weights is complete when this launch may start
 };
 
 int launch_linear_simt(const LinearArgs& a);
@@ -205,6 +206,8 @@ bool gemv_supported(const LinearArgs& a);
 size_t gemv_workspace_bytes(int bits, int64_t M, int64_t K, int64_t N, int layout);
 int launch_linear_gemv(const LinearArgs& a);
 int launch_linear_gemv_static(LinearArgs a);   // scratch in a file-scope device array
+size_t gemv_blocks_workspace_bytes(int64_t M, int64_t K);
+int launch_linear_gemv_blocks(const LinearArgs& a, int64_t* taken);   // 17 rows and more; rows it did not take are the caller's
 size_t gemv_prepared_bytes(int64_t M, int64_t K);            // 0: no prepared form for this (M, K)
 int launch_prepare_x(const float* x, int64_t M, int64_t K, void* prepared, cudaStream_t s);
 int launch_linear_gemv_prepared(const LinearArgs& a);        // a.workspace = prepared activations, a.x unused

@@ -621,3 +621,22 @@ def test_quantize_activations_int8_bit_exact(sgq, port, M, K):
     codes, scales = port.quantize_int8(x, cases.PER_ROW)
     assert np.array_equal(xq.cpu().numpy(), codes)
     assert sx.cpu().numpy().tobytes() == np.asarray(scales, np.float32).tobytes()
+
+
+@pytest.mark.parametrize("M,K", [(24, 768), (32, 4096), (40, 4096), (57, 4096), (48, 8192), (20, 256)])
+def test_batches_converted_in_front_match_their_blocks(sgq, M, K):
+    """17 .. 63 rows, INT4: one conversion launch for all blocks, or (scratch of one block only) one per block; blocks of 16 and
+    of 8 rows, with and without a remainder.  The same launches see the same planes, so the bits are the same."""
+    N = 272
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, device="cuda", generator=gen)
+    x[:, ::97] *= 30.0
+    q = sgq.quantize_int4(torch.randn(N, K, device="cuda", generator=gen) * 0.02, 32)
+    ws = sgq.Workspace(torch.device("cuda"))
+    blocks = torch.cat([sgq.quantized_matmul(x[m0:m0 + 16], q, None, layout=cases.LAYOUT_NK, path=sgq.PATH_GEMV, workspace=ws)
+                        for m0 in range(0, M, 16)])
+    one_block = max(sgq.linear_workspace_bytes(4, m, K, N, cases.LAYOUT_NK, sgq.PATH_GEMV) for m in (16, M % 16))
+    for limit in (None, one_block):
+        y = sgq.quantized_matmul(x, q, None, layout=cases.LAYOUT_NK, workspace=sgq.Workspace(torch.device("cuda")), workspace_limit=limit)
+        check_status(sgq)
+        assert torch.equal(y, blocks)
