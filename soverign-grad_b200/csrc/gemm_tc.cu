@@ -701,10 +701,25 @@ __global__ void __launch_bounds__(256) convert_x_bf16_kernel(const float* __rest
 constexpr int kExpandCtasPerSm = 2;
 constexpr int kReadyParts = 8;            // at most
 constexpr size_t kReadyBytes = 256;       // reserved behind the expanded weight for the counters
+
+// n / d for n < 2^31 by one multiplication: with 2^(s-1) < d <= 2^s and m = floor(2^(31+s) / d) + 1, m exceeds the exact
+// quotient by at most 1, and n * 1 / 2^(31+s) < 2^-s <= 1/d, too little to reach the next integer.  (The compiler's
+// division by a variable is about twenty instructions, and the kernel below needs two per eight elements.)
+struct FastDiv {
+    uint32_t d, m, s;
+    explicit FastDiv(uint32_t d_) : d(d_), m(0), s(0) {
+        while ((1ull << s) < d) ++s;
+        m = static_cast<uint32_t>((1ull << (31 + s)) / d + 1);          // at most 2^32 - 1 (d > 2^(s-1)), 2^31 + 1 for powers of two
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+        return static_cast<uint32_t>((static_cast<uint64_t>(n) * m) >> (31 + s));
+    }
+};
+
 template <int BITS, bool KN>
 __global__ void __maxnreg__(64)            // per SM quarter: 4 of these warps (4 x 64 x 32) beside 2 of the GEMM (2 x 128 x 32)
-expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ scales, uint32_t steps_per_scale, uint32_t N, uint32_t K,
-                      uint32_t parts, uint4* __restrict__ out, const float* __restrict__ x, uint32_t M, uint4* __restrict__ xout,
+expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ scales, FastDiv per_scale, FastDiv per_slice, uint32_t N,
+                      uint32_t K, uint32_t parts, uint4* __restrict__ out, const float* __restrict__ x, uint32_t M, uint4* __restrict__ xout,
                       uint32_t* __restrict__ ready) {
     pdl_launch_dependents();             // the GEMM behind this launch may take its places now; it waits on `ready`
     auto pk = [](float lo, float hi) {
@@ -712,11 +727,11 @@ expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ 
                (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << 16);
     };
     const uint32_t first = blockIdx.x * 256u + threadIdx.x, stride = gridDim.x * 256u;
-    const uint32_t row = K / 8, slice = row / parts;                     // steps per row of x (and of W [N,K]) / per row and slice
+    const uint32_t row = K / 8, slice = per_slice.d;                     // steps per row of x (and of W [N,K]) / per row and slice
     const uint32_t wslice = KN ? (K / parts) * (N / 8) : N * slice;      // steps of W per slice
     constexpr bool scaled = BITS == 4 || KN;                             // multiply here (else the epilogue does)
     auto step_of = [&](uint32_t v, uint32_t part) {                      // v-th step of the slice -> index in the whole tensor
-        const uint32_t r = v / slice;
+        const uint32_t r = per_slice(v);
         return r * row + part * slice + (v - r * slice);
     };
     auto expand = [&](uint32_t i, uint32_t lo, uint32_t hi, float sc) {
@@ -737,47 +752,53 @@ expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ 
         }
         out[i] = make_uint4(pk(v[0], v[1]), pk(v[2], v[3]), pk(v[4], v[5]), pk(v[6], v[7]));
     };
-    auto signal = [&](uint32_t part) {                                   // called by whole CTAs only
-        __threadfence();
+    // Called by whole CTAs only.  The barrier orders the CTA's stores before thread 0's fence, which makes all of them
+    // visible to the GPU before the count; the other threads go on to the next slice instead of waiting for their stores.
+    auto signal = [&](uint32_t part) {
         __syncthreads();
-        if (threadIdx.x == 0) atomicAdd(ready + part, 1u);
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(ready + part, 1u);
+        }
     };
+    // Four words and their scales per thread and pass, and the loads of the next pass, be it in this slice or the next,
+    // are issued before the current one is converted (before the slice's activations for the first): with two CTAs per SM
+    // the loads have to overlap the arithmetic inside a thread, and a slice that began with nothing on its way waited for
+    // memory twice (INT8 [4096,11008], 1000 rows: 47 us, now 37; INT4 [6144,2048], 4096 rows: 39, now 31).
+    uint32_t i[4], in[4];
+    uint32_t lo[4], hi[4], lon[4], hin[4];
+    float sc[4], scn[4];
+    auto fetch = [&](uint32_t v, uint32_t part, uint32_t (&ii)[4], uint32_t (&l)[4], uint32_t (&h)[4], float (&f)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t vq = v + q * stride, vv = vq < wslice ? vq : v;
+            ii[q] = KN ? part * wslice + vv : step_of(vv, part);
+            if (BITS == 4) {
+                l[q] = reinterpret_cast<const uint32_t*>(wq)[ii[q]];
+                h[q] = 0;
+            } else {
+                const uint2 w = reinterpret_cast<const uint2*>(wq)[ii[q]];
+                l[q] = w.x;
+                h[q] = w.y;
+            }
+            f[q] = scaled ? scales[per_scale(ii[q])] : 1.0f;              // a step never straddles groups or rows
+        }
+    };
+    if (first < wslice) fetch(first, 0, i, lo, hi, sc);
     for (uint32_t part = 0; part < parts; ++part) {
         const uint32_t xtotal = M * slice;
-        for (uint32_t v0 = blockIdx.x * 256u; v0 < xtotal; v0 += 2 * stride) {      // two chunks in flight per thread;
-            const uint32_t v = v0 + threadIdx.x;                                    // the trip count is the CTA's
-            const bool one = v < xtotal, two = v + stride < xtotal;
-            const uint32_t j0 = step_of(one ? v : 0, part), j1 = two ? step_of(v + stride, part) : j0;
+        for (uint32_t v = first; v < xtotal; v += 2 * stride) {                     // two chunks in flight per thread
+            const bool two = v + stride < xtotal;
+            const uint32_t j0 = step_of(v, part), j1 = two ? step_of(v + stride, part) : j0;
             const float4 a0 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j0)], b0 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j0) + 1];
             const float4 a1 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j1)], b1 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j1) + 1];
-            if (one) xout[j0] = make_uint4(pk(a0.x, a0.y), pk(a0.z, a0.w), pk(b0.x, b0.y), pk(b0.z, b0.w));
+            xout[j0] = make_uint4(pk(a0.x, a0.y), pk(a0.z, a0.w), pk(b0.x, b0.y), pk(b0.z, b0.w));
             if (two) xout[j1] = make_uint4(pk(a1.x, a1.y), pk(a1.z, a1.w), pk(b1.x, b1.y), pk(b1.z, b1.w));
         }
-        // Four words and their scales per thread and pass, and the loads of the next pass are issued before the
-        // current one is converted: with two CTAs per SM the loads have to overlap the arithmetic inside a thread.
-        uint32_t i[4], in[4];
-        uint32_t lo[4], hi[4], lon[4], hin[4];
-        float sc[4], scn[4];
-        auto fetch = [&](uint32_t v, uint32_t (&ii)[4], uint32_t (&l)[4], uint32_t (&h)[4], float (&f)[4]) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t vq = v + q * stride, vv = vq < wslice ? vq : v;
-                ii[q] = KN ? part * wslice + vv : step_of(vv, part);
-                if (BITS == 4) {
-                    l[q] = reinterpret_cast<const uint32_t*>(wq)[ii[q]];
-                    h[q] = 0;
-                } else {
-                    const uint2 w = reinterpret_cast<const uint2*>(wq)[ii[q]];
-                    l[q] = w.x;
-                    h[q] = w.y;
-                }
-                f[q] = scaled ? scales[ii[q] / steps_per_scale] : 1.0f;    // a step never straddles groups or rows
-            }
-        };
-        if (first < wslice) fetch(first, i, lo, hi, sc);
         for (uint32_t v = first; v < wslice; v += 4 * stride) {
             const uint32_t vn = v + 4 * stride;
-            if (vn < wslice) fetch(vn, in, lon, hin, scn);
+            if (vn < wslice) fetch(vn, part, in, lon, hin, scn);
+            else if (part + 1 < parts) fetch(first, part + 1, in, lon, hin, scn);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (q == 0 || v + q * stride < wslice) expand(i[q], lo[q], hi[q], sc[q]);
@@ -929,7 +950,8 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
         const int64_t wave = static_cast<int64_t>(sm_count()) * (beside ? kExpandCtasPerSm : 16);
         const int egrid = static_cast<int>(ceil_div(most, 1024) < wave ? ceil_div(most, 1024) : wave);
         const int64_t kblocks = a.K / 64;
-        int parts = beside ? kReadyParts : 1;
+        // Few slices where a thread has few passes: every slice ends in a pass that is partly empty.
+        int parts = !beside ? 1 : (wsteps >= 48LL * 4 * 256 * egrid ? kReadyParts : kReadyParts / 2);
         while (kblocks % parts) parts /= 2;
         if (most >= (1LL << 31) - 4LL * egrid * 256) {
             set_error("bf16 tensor-core path: more than 2^31 expansion steps");
@@ -942,13 +964,15 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
             p.sw = a.scales;
             p.sw_per_row = (a.scheme == SGQ_PER_ROW) ? 1 : 0;
         }
-        const uint32_t steps_per_scale =
-            a.bits == 4 ? static_cast<uint32_t>(a.group / 8) : (a.scheme == SGQ_PER_ROW ? static_cast<uint32_t>(a.N / 8) : UINT32_MAX);
+        // (one scale for all: more steps per scale than there are)
+        const FastDiv per_scale(a.bits == 4 ? static_cast<uint32_t>(a.group / 8 < (1LL << 31) ? a.group / 8 : (1LL << 31))
+                                            : (a.scheme == SGQ_PER_ROW && kn ? static_cast<uint32_t>(a.N / 8) : 1u << 31));
+        const FastDiv per_slice(static_cast<uint32_t>(a.K / 8 / parts));
         const auto kernel = a.bits == 4 ? (kn ? expand_ordered_kernel<4, true> : expand_ordered_kernel<4, false>)
                                         : (kn ? expand_ordered_kernel<8, true> : expand_ordered_kernel<8, false>);
         // the GEMM's CTA can only join an SM that runs under the same memory split
         prefer_max_shared(reinterpret_cast<const void*>(kernel));
-        kernel<<<egrid, 256, 0, a.stream>>>(static_cast<const uint8_t*>(a.wq), a.scales, steps_per_scale, static_cast<uint32_t>(a.N),
+        kernel<<<egrid, 256, 0, a.stream>>>(static_cast<const uint8_t*>(a.wq), a.scales, per_scale, per_slice, static_cast<uint32_t>(a.N),
                                             static_cast<uint32_t>(a.K), static_cast<uint32_t>(parts), reinterpret_cast<uint4*>(wt), a.x,
                                             static_cast<uint32_t>(a.M), reinterpret_cast<uint4*>(xb), ready);
         SGQ_LAUNCH_CHECK("expand_ordered_kernel");
