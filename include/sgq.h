@@ -77,10 +77,9 @@ enum {
     SGQ_PATH_TC_BF16 = 3, /* prefill: tcgen05 kind::f16 on bf16 activations and bf16 weights (INT4 with any group that is a
                              multiple of 8, or INT8; K % 64 == 0).
                              With the scratch sgq_linear_workspace_bytes() asks for, a launch in front expands the weight
-                             to bf16 [N,K] (INT4: code * scale in fp32, rounded once; INT8 stored [N,K]: the exact codes,
+                             to bf16 in the order it is stored in (INT4: code * scale in fp32, rounded once; INT8 stored [N,K]: the exact codes,
                              scale applied in fp32 afterwards) and both operands reach the tensor cores by TMA; weights
-                             stored [K,N] (N % 32 == 0) are transposed by that launch.  For weights stored [N,K] and
-                             with sgq_set_stream_overlap on, the GEMM starts while that launch is still running: the
+                             stored [K,N] need N % 32 == 0.  The GEMM starts while that launch is still running: the
                              expansion goes slice of K by slice of K and counts finished slices in the last 256 bytes of
                              the scratch, which the GEMM's loads wait on (bounded).  With scratch for the activations
                              only (M * K * 2 bytes, rounded up to 256), INT4 g=32 and INT8 weights stored [N,K] are dequantized tile by tile in
