@@ -160,10 +160,10 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 float* fptr(const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 
 // bias as N fp32 values, or an empty tensor
-at::Tensor bias_of(PyObject* o, int64_t N, const char* msg) {
+at::Tensor bias_of(PyObject* o, int64_t N) {
     if (o == Py_None) return at::Tensor();
     at::Tensor b = f32_cuda(o);
-    if (b.numel() != N && msg) raise(PyExc_RuntimeError, msg);
+    if (b.numel() != N) raise(PyExc_RuntimeError, "Incompatible shapes for broadcasting!");      // src/ops.cpp:60
     return b;
 }
 
@@ -177,7 +177,7 @@ PyObject* quantized_matmul(PyObject* const* a, Py_ssize_t n) {
     if (q.dims != 2) raise(PyExc_RuntimeError, "matmul currently requires 2D tensors!");                     // src/ops.cpp:380-382
     const int64_t K = layout == SGQ_LAYOUT_KN ? q.rows : q.cols, N = layout == SGQ_LAYOUT_KN ? q.cols : q.rows, M = x.size(0);
     if (x.size(1) != K) raise(PyExc_RuntimeError, "Matrix inner dimensions must match for matmul!");         // src/ops.cpp:387-389
-    const at::Tensor bias = bias_of(a[2], N, "Incompatible shapes for broadcasting!");                      // src/ops.cpp:60
+    const at::Tensor bias = bias_of(a[2], N);
     at::Tensor out;
     int64_t ldy = N;
     if (a[5] == Py_None) {
@@ -231,15 +231,22 @@ PyObject* backward_x(PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(dx));
 }
 
-// linear_w8a8(x, q, bias, want_parts)
+// linear_w8a8(x, q, bias, want_parts).  Every shape is checked here, before the device: the library below sees pointers and
+// M, K, N only, and a narrower x, packed INT4 codes or a short bias would be read past their end.
 PyObject* linear_w8a8(PyObject* const* a, Py_ssize_t n) {
     if (n != 4) raise(PyExc_TypeError, "linear_w8a8 takes four arguments");
-    const at::Tensor x = f32_cuda(a[0]);
+    const at::Tensor& given = as_tensor(a[0]);
     const Quantized q(a[1]);
-    const int64_t N = q.rows, K = q.cols, M = x.size(0);
-    const at::Tensor bias = bias_of(a[2], N, nullptr);
+    if (given.dim() != 2 || q.dims != 2) raise(PyExc_RuntimeError, "matmul currently requires 2D tensors!");
+    if (q.bits != 8) raise(PyExc_RuntimeError, "linear_w8a8 needs an INT8 weight stored [N,K]");
+    const int64_t N = q.rows, K = q.cols, M = given.size(0);
+    if (given.size(1) != K) raise(PyExc_RuntimeError, "Matrix inner dimensions must match for matmul!");
+    if (a[2] != Py_None && as_tensor(a[2]).numel() != N) raise(PyExc_RuntimeError, "Incompatible shapes for broadcasting!");
+    const int parts_asked = PyObject_IsTrue(a[3]);
+    if (parts_asked < 0) throw PythonError();
+    const at::Tensor x = f32_cuda(a[0]), bias = bias_of(a[2], N);
     at::Tensor y = empty({M, N}, at::kFloat, x), xq, sx, acc;
-    const bool parts = PyObject_IsTrue(a[3]) == 1;
+    const bool parts = parts_asked == 1;
     if (parts) {
         xq = empty({M, K}, at::kChar, x);
         sx = empty({M}, at::kFloat, x);

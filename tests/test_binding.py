@@ -1,0 +1,44 @@
+"""The native calls of the Python package (csrc/torch_binding.cpp): what they refuse, and what they read of the objects they
+are given.  Shapes are checked before the device, so the refusals need no GPU."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def sgq():
+    from __graft_entry__ import load_package
+    return load_package()
+
+
+def int8_weight(sgq, shape):
+    n = 1
+    for d in shape:
+        n *= d
+    return sgq.QuantizedTensor(torch.zeros(shape, dtype=torch.int8), torch.ones(shape[0]), sgq.PER_ROW, shape, n, 8)
+
+
+def test_w8a8_refuses_weights_that_are_not_int8_matrices(sgq):
+    """A weight of three dimensions must not be read as the matrix of its first two."""
+    for shape in ((2, 16, 4), (32,), (2, 16, 1, 1)):
+        with pytest.raises(RuntimeError, match="2D"):
+            sgq.linear_w8a8(torch.zeros(3, 16), int8_weight(sgq, shape))
+    packed = sgq.QuantizedTensor(torch.zeros(2 * 16 // 2, dtype=torch.uint8), torch.ones(1), sgq.PER_TENSOR, (2, 16), 32, 4)
+    with pytest.raises(RuntimeError, match="INT8"):
+        sgq.linear_w8a8(torch.zeros(3, 16), packed)
+
+
+def test_w8a8_refuses_operands_that_do_not_fit_the_weight(sgq):
+    """Narrower activations or a short bias would be read past their end."""
+    q = int8_weight(sgq, (8, 32))
+    for x in (torch.zeros(32), torch.zeros(1, 3, 32)):
+        with pytest.raises(RuntimeError, match="2D"):
+            sgq.linear_w8a8(x, q)
+    for k in (16, 48):
+        with pytest.raises(RuntimeError, match="inner dimensions"):
+            sgq.linear_w8a8(torch.zeros(3, k), q)
+    for n in (1, 7, 9):
+        with pytest.raises(RuntimeError, match="broadcasting"):
+            sgq.linear_w8a8(torch.zeros(3, 32), q, torch.zeros(n))
+    with pytest.raises(ValueError, match="CUDA"):                     # everything fits: the device is what is left to refuse
+        sgq.linear_w8a8(torch.zeros(3, 32), q, torch.zeros(8))
