@@ -73,7 +73,7 @@ enum {
                              dominates its 32), fp32 scaling and accumulation; any activation distribution stays
                              within ~1e-4 of the reference's fp32 forward (bound 1e-3); a row with a
                              NaN or Inf activation yields a NaN output row.  [K,N] (the reference module's layout):
-                             fp32 throughout */
+                             fp32 throughout, +-Inf and NaN per output as the reference's chain gives them */
     SGQ_PATH_TC_BF16 = 3, /* prefill: tcgen05 kind::f16 on bf16 activations and bf16 weights (INT4 with any group that is a
                              multiple of 8, or INT8; K % 64 == 0).
                              With the scratch sgq_linear_workspace_bytes() asks for, a launch in front expands the weight

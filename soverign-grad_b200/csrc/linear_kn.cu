@@ -28,7 +28,11 @@
 // number and one subtraction; a second kernel adds the slices in ascending order and the bias.
 //
 // fp32 throughout in either form; the summation order differs from the reference's single chain, the result is inside the
-// 1e-3 contract.  (A NaN or Inf activation gives a NaN output row in the tensor-core form.)
+// 1e-3 contract.  The split holds away from the ends of the exponent range only: the remainders of an Inf, and of a finite
+// factor above bf16's largest value, are Inf - Inf, and those of a factor below about 2^-110 end under bf16's smallest.  The
+// first makes every output of its row NaN, the second leaves outputs near zero, so the epilogue recognises both by the sum
+// itself and forms such an output again as the plain chain of fp32 multiply-adds (kn_chain4): +-Inf and NaN per output as
+// in the reference, and no loss for vanishing rows.
 #include "sgq_common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -88,6 +92,8 @@ struct KnMmaParams {
     int M;
     int64_t K, N;
     int early;               // weights may be requested before the dependency wait (overlapped launches)
+    const float* x;          // operands by address, for kn_chain4
+    const uint8_t* wq;
 };
 
 __device__ __forceinline__ void kn_cp_async_16(uint32_t dst, const void* src, int bytes) {
@@ -122,9 +128,38 @@ __device__ __forceinline__ void split3(float p0, float p1, uint32_t (&part)[3]) 
     }
 }
 
+// Whether a sum (without the bias) may come from factors that the split does not hold exactly: not finite, or below 2^-90 and
+// not zero.  (Factors below 2^-110, or 2^-117 where remainders under 2^-126 count as zero, are wrong by at most 2^-126: 2^13
+// of them times a code of 8 are 2^-110, a millionth of the smallest sum that passes.  A row of zeros is exact.)
+__device__ __forceinline__ bool kn_sum_suspect(float v) {
+    const float a = fabsf(v);
+    return !(a >= 8.07793567e-28f && a <= 3.402823466e+38f) && a != 0.0f;      // true for NaN
+}
+
+// Outputs (m, n .. n + 3) as one chain of fp32 multiply-adds each, in ascending k.  A call of its own (not inlined): it runs for
+// rows at the ends of the exponent range only, and its registers are not the kernel's.
+template <int BITS>
+__device__ __noinline__ float4 kn_chain4(const KnMmaParams& p, int m, int64_t n) {
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const float* x = p.x + static_cast<int64_t>(m) * p.K;
+    const int64_t row_bytes = BITS == 4 ? p.N / 2 : p.N;
+    const uint8_t* w = p.wq + (BITS == 4 ? n / 2 : n);
+    const int64_t per_row = BITS == 4 ? p.N / p.group : 1;
+    const float* s = p.scales + (BITS == 4 ? n / p.group : 0);          // a group holds whole runs of 32 features
+#pragma unroll 4
+    for (int64_t k = 0; k < p.K; ++k) {
+        const float f = x[k] * (p.scale_mode == 2 ? s[0] : s[k * per_row]);
+        const uint32_t c = BITS == 4 ? *reinterpret_cast<const uint16_t*>(w + k * row_bytes) : *reinterpret_cast<const uint32_t*>(w + k * row_bytes);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            acc[j] = fmaf(f, static_cast<float>(static_cast<int>(c << (32 - BITS - BITS * j)) >> (32 - BITS)), acc[j]);
+    }
+    return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 template <int BITS, int T, int NBW>
 __global__ void __launch_bounds__(kMmaThreads, 2)
-kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const KnMmaParams p) {
+kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ KnMmaParams p) {
     using C = KnCfg<BITS, T, NBW>;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -448,6 +483,7 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         }
         const int64_t n = n0 + c;
         if (n < p.N) {                                       // N % 4 == 0
+            if (kn_sum_suspect(v.x) || kn_sum_suspect(v.y) || kn_sum_suspect(v.z) || kn_sum_suspect(v.w)) v = kn_chain4<BITS>(p, m, n);
             if (p.bias) { v.x += p.bias[n]; v.y += p.bias[n + 1]; v.z += p.bias[n + 2]; v.w += p.bias[n + 3]; }
             float* dst = p.y + static_cast<int64_t>(m) * p.ldy + n;
             if (p.vec_y) {
@@ -506,6 +542,7 @@ int launch_mma(const LinearArgs& a, int slices) {
     p.bias = a.bias; p.y = a.y; p.ldy = a.ldy; p.M = static_cast<int>(a.M); p.K = a.K; p.N = a.N;
     p.vec_y = aligned(a.y, 16) && (a.ldy % 4) == 0 ? 1 : 0;
     p.early = stream_overlap_enabled() ? 1 : 0;
+    p.x = a.x; p.wq = static_cast<const uint8_t*>(a.wq);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(a.N, C::kFeatures)), static_cast<unsigned>(slices));
     cfg.blockDim = dim3(kMmaThreads);

@@ -47,3 +47,49 @@ def test_kn_tensor_core_decode(sgq, port, M, K, N, group):
     xd[M - 1, K // 2] = float("nan")
     y = sgq.quantized_matmul(xd, runs[0][0], None, layout=cases.LAYOUT_KN, workspace=ws)
     assert torch.isnan(y[M - 1]).all() and torch.isfinite(y[: M - 1]).all()
+
+
+EXTREMES = ["inf", "-inf", "both", "nan", "huge", "tiny"]
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("kind", EXTREMES)
+def test_kn_decode_non_finite_and_extreme_activations(sgq, M, kind):
+    """Factors x * s that the three bf16 parts do not hold: Inf, NaN, a finite one above bf16's largest value, and a row of
+    factors whose parts lie below bf16's smallest.  Codes with zeros among them, every scale exactly 1; +-Inf and NaN per
+    output as in the reference's fp32 chain, the other rows the same bits as without that row."""
+    K, N = 520, 288
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    w = torch.randint(-7, 8, (K, N), device="cuda", generator=gen).float()
+    w[:, ::32] = 7.0                                        # every scale is exactly 1
+    w8 = torch.randint(-127, 128, (K, N), device="cuda", generator=gen).float() * (torch.rand(K, N, device="cuda", generator=gen) < 0.9)
+    w8[:, 0] = 127.0
+    x = torch.randn(M, K, device="cuda", generator=gen)
+    clean, m = x.clone(), M - 1
+    if kind == "huge":
+        x[m] = 0.0
+        x[m, 77] = 3.4e38                                   # above the largest bf16 value
+    elif kind == "tiny":
+        x[m] *= 1e-37
+    elif kind == "both":
+        x[m, 3], x[m, 400] = float("inf"), float("-inf")
+    else:
+        x[m, 77] = float(kind)
+    ws = sgq.Workspace(x.device)
+    runs = [(sgq.quantize_int4(w, 32), w), (sgq.quantize_int8(w8, sgq.PER_ROW), w8), (sgq.quantize_int8(w8, sgq.PER_TENSOR), w8)]
+    bias = torch.randn(N, device="cuda", generator=gen)
+    for q, deq in runs:
+        for b in (None, bias):
+            y = sgq.quantized_matmul(x, q, b, layout=sgq.LAYOUT_KN, path=sgq.PATH_GEMV, workspace=ws)
+            y_clean = sgq.quantized_matmul(clean, q, b, layout=sgq.LAYOUT_KN, path=sgq.PATH_GEMV, workspace=ws)
+            assert sgq.device_status() == 0
+            assert torch.equal(y[:m], y_clean[:m])          # rows do not mix
+            terms = x[m].double()[:, None] * deq.double()
+            want = terms.sum(0) + (0.0 if b is None else b.double())
+            got, want32 = y[m], want.float()
+            assert torch.equal(torch.isnan(got), torch.isnan(want32)), kind
+            assert torch.equal(torch.isinf(got), torch.isinf(want32)) and torch.equal(got[got.isinf()], want32[want32.isinf()])
+            fin = torch.isfinite(want32)
+            mag = terms.abs().sum(0) + (0.0 if b is None else b.abs().double())
+            err = (got.double() - want).abs()               # one rounding of the running sum per term, or of the smallest subnormal
+            assert bool((err <= mag * (K + 8) * 2.0 ** -23 + K * 2.0 ** -149)[fin].all()), (kind, float((err / mag)[fin].max()))
