@@ -574,9 +574,18 @@ int launch_mma_rows(const LinearArgs& a, const KnSplit& sp) {
     return launch_mma_nb<BITS, 6>(a, sp);
 }
 
-// TMA needs rows that are multiples of 16 bytes; a warp's 32 features must lie in one INT4 group
+// Whether the output rows and x share memory (a caller that multiplies in place, K == N).
+bool output_overlaps_x(const LinearArgs& a) {
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(a.x), y0 = reinterpret_cast<uintptr_t>(a.y);
+    const uintptr_t x1 = x0 + static_cast<uintptr_t>(a.M * a.K) * 4, y1 = y0 + static_cast<uintptr_t>((a.M - 1) * a.ldy + a.N) * 4;
+    return x0 < y1 && y0 < x1;
+}
+
+// TMA needs rows that are multiples of 16 bytes; a warp's 32 features must lie in one INT4 group.  One launch reads x and
+// stores y, a cluster storing its columns while others still load x: an output that overlaps x goes to the any-shape form,
+// whose first launch reads the rows of a pass and whose second stores them.
 bool kn_mma_supported(const LinearArgs& a) {
-    return (a.K % 4) == 0 && aligned(a.x, 16) && (a.bits == 8 || ((a.N % 32) == 0 && (a.group % 32) == 0)) && a.K < (1LL << 24);
+    return !output_overlaps_x(a) && (a.K % 4) == 0 && aligned(a.x, 16) && (a.bits == 8 || ((a.N % 32) == 0 && (a.group % 32) == 0)) && a.K < (1LL << 24);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

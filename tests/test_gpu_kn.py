@@ -93,3 +93,26 @@ def test_kn_decode_non_finite_and_extreme_activations(sgq, M, kind):
             mag = terms.abs().sum(0) + (0.0 if b is None else b.abs().double())
             err = (got.double() - want).abs()               # one rounding of the running sum per term, or of the smallest subnormal
             assert bool((err <= mag * (K + 8) * 2.0 ** -23 + K * 2.0 ** -149)[fin].all()), (kind, float((err / mag)[fin].max()))
+
+
+@pytest.mark.parametrize("M", [1, 3, 16, 40, 128])
+def test_kn_forward_in_place(sgq, M):
+    """The output may be the activations' own buffer (K == N): every launch that stores it starts behind the ones that read x.
+    Up to 63 rows the bits are those of the any-shape form, which is what an overlapping output takes; a view that starts four
+    bytes off a row is one that the tensor-core form does not take either."""
+    K = N = 512
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=gen)
+    w = torch.randn(K, N, device="cuda", generator=gen) * 0.05
+    ws = sgq.Workspace(x.device)
+    for q in (sgq.quantize_int4(w, 32), sgq.quantize_int8(w, sgq.PER_ROW)):
+        apart = sgq.quantized_matmul(x, q, workspace=ws)
+        shifted = torch.empty(M * K + 1, device="cuda")[1:].view(M, K)
+        shifted.copy_(x)
+        other = sgq.quantized_matmul(shifted, q, workspace=ws) if M < 64 else apart
+        for _ in range(20):
+            buf = x.clone()
+            got = sgq.quantized_matmul(buf, q, out=buf, workspace=ws)
+            assert got is buf and torch.equal(got, other)
+        assert rel_err(got.cpu().numpy(), apart.cpu().numpy()) <= 1e-5
+    assert sgq.device_status() == 0
