@@ -697,7 +697,8 @@ __global__ void __launch_bounds__(256) convert_x_bf16_kernel(const float* __rest
 // for the GEMM's CTA on every SM, and the work is ordered by `parts` equal slices of K: slice 0 of x, slice 0 of W,
 // slice 1 of x, ...  ready[q] counts the CTAs that have finished slice q of both; a CTA counts itself after a fence
 // behind all of its stores, so a reader that sees gridDim.x in ready[q] (acquire load) may read slices 0 .. q.  The
-// counters must be zero at launch.  Indices are 32-bit: the host refuses a weight of 2^31 steps or more.
+// counters must be zero at launch.  Indices are 32-bit with FastDiv; a [K,N] weight or its activations of 2^31 steps or more
+// (2^34 elements) take the 64-bit form, WideDiv.
 constexpr int kExpandCtasPerSm = 2;
 constexpr int kReadyParts = 8;            // at most
 constexpr size_t kReadyBytes = 256;       // reserved behind the expanded weight for the counters
@@ -706,6 +707,7 @@ constexpr size_t kReadyBytes = 256;       // reserved behind the expanded weight
 // quotient by at most 1, and n * 1 / 2^(31+s) < 2^-s <= 1/d, too little to reach the next integer.  (The compiler's
 // division by a variable is about twenty instructions, and the kernel below needs two per eight elements.)
 struct FastDiv {
+    using Index = uint32_t;
     uint32_t d, m, s;
     explicit FastDiv(uint32_t d_) : d(d_), m(0), s(0) {
         while ((1ull << s) < d) ++s;
@@ -716,9 +718,16 @@ struct FastDiv {
     }
 };
 
-template <int BITS, bool KN>
+struct WideDiv {
+    using Index = uint64_t;
+    uint64_t d;
+    explicit WideDiv(uint64_t d_) : d(d_) {}
+    __device__ __forceinline__ uint64_t operator()(uint64_t n) const { return n / d; }
+};
+
+template <int BITS, bool KN, typename Div>
 __global__ void __maxnreg__(64)            // per SM quarter: 4 of these warps (4 x 64 x 32) beside 2 of the GEMM (2 x 128 x 32)
-expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ scales, FastDiv per_scale, FastDiv per_slice, uint32_t N,
+expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ scales, Div per_scale, Div per_slice, uint32_t N,
                       uint32_t K, uint32_t parts, uint4* __restrict__ out, const float* __restrict__ x, uint32_t M, uint4* __restrict__ xout,
                       uint32_t* __restrict__ ready) {
     pdl_launch_dependents();             // the GEMM behind this launch may take its places now; it waits on `ready`
@@ -726,15 +735,16 @@ expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ 
         return static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(lo))) |
                (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(hi))) << 16);
     };
-    const uint32_t first = blockIdx.x * 256u + threadIdx.x, stride = gridDim.x * 256u;
-    const uint32_t row = K / 8, slice = per_slice.d;                     // steps per row of x (and of W [N,K]) / per row and slice
-    const uint32_t wslice = KN ? (K / parts) * (N / 8) : N * slice;      // steps of W per slice
+    using Index = typename Div::Index;
+    const Index first = blockIdx.x * 256u + threadIdx.x, stride = gridDim.x * 256u;
+    const Index row = K / 8, slice = per_slice.d;                        // steps per row of x (and of W [N,K]) / per row and slice
+    const Index wslice = KN ? (K / parts) * static_cast<Index>(N / 8) : N * slice;      // steps of W per slice
     constexpr bool scaled = BITS == 4 || KN;                             // multiply here (else the epilogue does)
-    auto step_of = [&](uint32_t v, uint32_t part) {                      // v-th step of the slice -> index in the whole tensor
-        const uint32_t r = per_slice(v);
+    auto step_of = [&](Index v, uint32_t part) {                      // v-th step of the slice -> index in the whole tensor
+        const Index r = per_slice(v);
         return r * row + part * slice + (v - r * slice);
     };
-    auto expand = [&](uint32_t i, uint32_t lo, uint32_t hi, float sc) {
+    auto expand = [&](Index i, uint32_t lo, uint32_t hi, float sc) {
         float v[8];
         if (BITS == 4) {
 #pragma unroll
@@ -765,13 +775,13 @@ expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ 
     // are issued before the current one is converted (before the slice's activations for the first): with two CTAs per SM
     // the loads have to overlap the arithmetic inside a thread, and a slice that began with nothing on its way waited for
     // memory twice (INT8 [4096,11008], 1000 rows: 47 us, now 37; INT4 [6144,2048], 4096 rows: 39, now 31).
-    uint32_t i[4], in[4];
+    Index i[4], in[4];
     uint32_t lo[4], hi[4], lon[4], hin[4];
     float sc[4], scn[4];
-    auto fetch = [&](uint32_t v, uint32_t part, uint32_t (&ii)[4], uint32_t (&l)[4], uint32_t (&h)[4], float (&f)[4]) {
+    auto fetch = [&](Index v, uint32_t part, Index (&ii)[4], uint32_t (&l)[4], uint32_t (&h)[4], float (&f)[4]) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t vq = v + q * stride, vv = vq < wslice ? vq : v;
+            const Index vq = v + q * stride, vv = vq < wslice ? vq : v;
             ii[q] = KN ? part * wslice + vv : step_of(vv, part);
             if (BITS == 4) {
                 l[q] = reinterpret_cast<const uint32_t*>(wq)[ii[q]];
@@ -786,17 +796,17 @@ expand_ordered_kernel(const uint8_t* __restrict__ wq, const float* __restrict__ 
     };
     if (first < wslice) fetch(first, 0, i, lo, hi, sc);
     for (uint32_t part = 0; part < parts; ++part) {
-        const uint32_t xtotal = M * slice;
-        for (uint32_t v = first; v < xtotal; v += 2 * stride) {                     // two chunks in flight per thread
+        const Index xtotal = M * slice;
+        for (Index v = first; v < xtotal; v += 2 * stride) {                     // two chunks in flight per thread
             const bool two = v + stride < xtotal;
-            const uint32_t j0 = step_of(v, part), j1 = two ? step_of(v + stride, part) : j0;
+            const Index j0 = step_of(v, part), j1 = two ? step_of(v + stride, part) : j0;
             const float4 a0 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j0)], b0 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j0) + 1];
             const float4 a1 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j1)], b1 = reinterpret_cast<const float4*>(x)[2 * static_cast<size_t>(j1) + 1];
             xout[j0] = make_uint4(pk(a0.x, a0.y), pk(a0.z, a0.w), pk(b0.x, b0.y), pk(b0.z, b0.w));
             if (two) xout[j1] = make_uint4(pk(a1.x, a1.y), pk(a1.z, a1.w), pk(b1.x, b1.y), pk(b1.z, b1.w));
         }
-        for (uint32_t v = first; v < wslice; v += 4 * stride) {
-            const uint32_t vn = v + 4 * stride;
+        for (Index v = first; v < wslice; v += 4 * stride) {
+            const Index vn = v + 4 * stride;
             if (vn < wslice) fetch(vn, part, in, lon, hin, scn);
             else if (part + 1 < parts) fetch(first, part + 1, in, lon, hin, scn);
 #pragma unroll
@@ -953,7 +963,9 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
         // Few slices where a thread has few passes: every slice ends in a pass that is partly empty.
         int parts = !beside ? 1 : (wsteps >= 48LL * 4 * 256 * egrid ? kReadyParts : kReadyParts / 2);
         while (kblocks % parts) parts /= 2;
-        if (most >= (1LL << 31) - 4LL * egrid * 256) {
+        // 32-bit indices hold up to 2^31 steps and what the last pass adds to them; weights stored [N,K] end there
+        const bool wide = most >= (1LL << 31) - 4LL * egrid * 256;
+        if (wide && !kn) {
             set_error("bf16 tensor-core path: more than 2^31 expansion steps");
             return SGQ_ERR_UNSUPPORTED;
         }
@@ -965,16 +977,25 @@ int launch_linear_tc_bf16(const LinearArgs& a) {
             p.sw_per_row = (a.scheme == SGQ_PER_ROW) ? 1 : 0;
         }
         // (one scale for all: more steps per scale than there are)
-        const FastDiv per_scale(a.bits == 4 ? static_cast<uint32_t>(a.group / 8 < (1LL << 31) ? a.group / 8 : (1LL << 31))
-                                            : (a.scheme == SGQ_PER_ROW && kn ? static_cast<uint32_t>(a.N / 8) : 1u << 31));
-        const FastDiv per_slice(static_cast<uint32_t>(a.K / 8 / parts));
-        const auto kernel = a.bits == 4 ? (kn ? expand_ordered_kernel<4, true> : expand_ordered_kernel<4, false>)
-                                        : (kn ? expand_ordered_kernel<8, true> : expand_ordered_kernel<8, false>);
-        // the GEMM's CTA can only join an SM that runs under the same memory split
-        prefer_max_shared(reinterpret_cast<const void*>(kernel));
-        kernel<<<egrid, 256, 0, a.stream>>>(static_cast<const uint8_t*>(a.wq), a.scales, per_scale, per_slice, static_cast<uint32_t>(a.N),
-                                            static_cast<uint32_t>(a.K), static_cast<uint32_t>(parts), reinterpret_cast<uint4*>(wt), a.x,
-                                            static_cast<uint32_t>(a.M), reinterpret_cast<uint4*>(xb), ready);
+        const int64_t scale_steps = a.bits == 4 ? a.group / 8 : (a.scheme == SGQ_PER_ROW && kn ? a.N / 8 : most + 1);
+        const int64_t slice_steps = a.K / 8 / parts;
+        auto run = [&](auto kernel, auto per_scale, auto per_slice) {
+            // the GEMM's CTA can only join an SM that runs under the same memory split
+            prefer_max_shared(reinterpret_cast<const void*>(kernel));
+            kernel<<<egrid, 256, 0, a.stream>>>(static_cast<const uint8_t*>(a.wq), a.scales, per_scale, per_slice, static_cast<uint32_t>(a.N),
+                                                static_cast<uint32_t>(a.K), static_cast<uint32_t>(parts), reinterpret_cast<uint4*>(wt), a.x,
+                                                static_cast<uint32_t>(a.M), reinterpret_cast<uint4*>(xb), ready);
+        };
+        if (wide) {
+            const WideDiv per_scale(static_cast<uint64_t>(scale_steps)), per_slice(static_cast<uint64_t>(slice_steps));
+            if (a.bits == 4) run(expand_ordered_kernel<4, true, WideDiv>, per_scale, per_slice);
+            else run(expand_ordered_kernel<8, true, WideDiv>, per_scale, per_slice);
+        } else {
+            const FastDiv per_scale(static_cast<uint32_t>(scale_steps < (1LL << 31) ? scale_steps : (1LL << 31)));
+            const FastDiv per_slice(static_cast<uint32_t>(slice_steps));
+            if (a.bits == 4) run(kn ? expand_ordered_kernel<4, true, FastDiv> : expand_ordered_kernel<4, false, FastDiv>, per_scale, per_slice);
+            else run(kn ? expand_ordered_kernel<8, true, FastDiv> : expand_ordered_kernel<8, false, FastDiv>, per_scale, per_slice);
+        }
         SGQ_LAUNCH_CHECK("expand_ordered_kernel");
         p.b_mn = kn ? 1 : 0;
         p.ready = ready;

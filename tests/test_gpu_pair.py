@@ -48,3 +48,23 @@ def test_pair_gemm_edges(sgq, M, K, N):
                 y = sgq.quantized_matmul(x, q, bias, layout=layout, path=sgq.PATH_TC_BF16, workspace=ws)
                 assert sgq.device_status() == 0
                 check(y if bias is None else y.double() - bias.double(), xb, wf, K + (0 if bias is None else 4096))
+
+
+def test_expansion_of_2_31_steps(sgq):
+    """A [K,N] weight of 2^34 codes: 2^31 steps of eight, one more than 32-bit indices hold.  x in {-1, 0, 1} and scales that are
+    powers of two from 1/2 to 4: every product is a multiple of 1/2 and the sums stay below 2^23, so fp32 holds them exactly."""
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB of device memory")
+    K = N = 1 << 17
+    M, group = 64, 128
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    codes = torch.randint(0, 256, (K * N // 2,), dtype=torch.uint8, device="cuda", generator=gen)
+    scales = torch.exp2(torch.randint(-1, 3, (K * N // group,), device="cuda", generator=gen, dtype=torch.int32).float())
+    q = sgq.QuantizedTensor(codes, scales, sgq.PER_TENSOR, (K, N), group, 4)
+    x = torch.randint(-1, 2, (M, K), device="cuda", generator=gen, dtype=torch.int32).float()
+    y = sgq.quantized_matmul(x, q, path=sgq.PATH_TC_BF16)
+    assert sgq.device_status() == 0
+    for n in (0, 1, 127, 128, 65535, 65536, 100001, N - 130, N - 1):
+        nibble = (codes.view(K, N // 2)[:, n // 2] >> (4 * (n % 2))) & 0xF
+        column = ((nibble.int() ^ 8) - 8).double() * scales.view(K, N // group)[:, n // group].double()
+        assert torch.equal(y[:, n].double(), x.double() @ column), n
