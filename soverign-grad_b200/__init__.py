@@ -185,9 +185,6 @@ class QuantizedTensor:
         return out
 
 
-_native.set_classes(SgqError, QuantizedTensor)
-
-
 def quantize_int8(x: torch.Tensor, scheme: int = PER_ROW) -> QuantizedTensor:
     """quantization::quantize_int8 (src/quantization.cpp:11-78)."""
     return _native.quantize_int8(x, scheme)
@@ -225,6 +222,9 @@ class Workspace:
         if self.buf is None or self.buf.numel() < nbytes:
             self.buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         return self.buf
+
+
+_native.set_classes(SgqError, QuantizedTensor, Workspace)
 
 
 def quantized_matmul(x: torch.Tensor, q: QuantizedTensor, bias: Optional[torch.Tensor] = None, *, layout: int = LAYOUT_KN,

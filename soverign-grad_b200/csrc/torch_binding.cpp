@@ -26,6 +26,7 @@ namespace {
 
 PyObject* g_error_class = nullptr;      // SgqError(status, what, detail)
 PyObject* g_tensor_class = nullptr;     // QuantizedTensor(qdata, scales, scheme, original_shape, group_size, bits)
+PyObject* g_workspace_class = nullptr;  // Workspace: .buf, .get(nbytes)
 
 PyObject *s_qdata, *s_scales, *s_scheme, *s_shape, *s_group, *s_bits, *s_buf, *s_get;
 
@@ -110,7 +111,9 @@ struct Quantized {
     int scheme_now() const { return scheme == SGQ_PER_TENSOR || scales.numel() == 1 ? SGQ_PER_TENSOR : SGQ_PER_ROW; }
 };
 
-// The scratch of a call: the caller's Workspace (grown by its own get()) or a buffer of this call.
+// The scratch of a call: what the caller's workspace gives for `need` bytes (None: nothing), or a buffer of this call.  The
+// package's own Workspace is read directly while its buffer is large enough; any other object, a class derived from it
+// included, is asked through its get().
 struct Scratch {
     at::Tensor buf;
     void* ptr = nullptr;
@@ -120,15 +123,19 @@ struct Scratch {
         if (workspace == Py_None) {
             buf = empty({static_cast<int64_t>(need)}, at::kByte, like);
         } else {
-            Ref b(PyObject_GetAttr(workspace, s_buf));
-            if (!b) throw PythonError();
-            if (b.p == Py_None || static_cast<size_t>(as_tensor(b.p).numel()) < need) {
-                Ref n(PyLong_FromSize_t(need));
-                Ref grown(n ? PyObject_CallMethodOneArg(workspace, s_get, n.p) : nullptr);
-                if (!grown) throw PythonError();
-                buf = as_tensor(grown.p);
-            } else {
+            Ref b;
+            if (reinterpret_cast<PyObject*>(Py_TYPE(workspace)) == g_workspace_class) {
+                b.p = PyObject_GetAttr(workspace, s_buf);
+                if (!b) throw PythonError();
+            }
+            if (b && b.p != Py_None && static_cast<size_t>(as_tensor(b.p).numel()) >= need) {
                 buf = as_tensor(b.p);
+            } else {
+                Ref n(PyLong_FromSize_t(need));
+                Ref given(n ? PyObject_CallMethodOneArg(workspace, s_get, n.p) : nullptr);
+                if (!given) throw PythonError();
+                if (given.p == Py_None) return;
+                buf = as_tensor(given.p);
             }
         }
         ptr = buf.data_ptr();
@@ -337,15 +344,15 @@ PyObject* dequantize(PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(out));
 }
 
-// set_classes(SgqError, QuantizedTensor)
+// set_classes(SgqError, QuantizedTensor, Workspace)
 PyObject* set_classes(PyObject* const* a, Py_ssize_t n) {
-    if (n != 2) raise(PyExc_TypeError, "set_classes takes two arguments");
-    Py_INCREF(a[0]);
-    Py_INCREF(a[1]);
-    Py_XDECREF(g_error_class);
-    Py_XDECREF(g_tensor_class);
-    g_error_class = a[0];
-    g_tensor_class = a[1];
+    if (n != 3) raise(PyExc_TypeError, "set_classes takes three arguments");
+    PyObject** const classes[] = {&g_error_class, &g_tensor_class, &g_workspace_class};
+    for (int i = 0; i < 3; ++i) {
+        Py_INCREF(a[i]);
+        Py_XDECREF(*classes[i]);
+        *classes[i] = a[i];
+    }
     Py_RETURN_NONE;
 }
 

@@ -42,3 +42,37 @@ def test_w8a8_refuses_operands_that_do_not_fit_the_weight(sgq):
             sgq.linear_w8a8(torch.zeros(3, 32), q, torch.zeros(n))
     with pytest.raises(ValueError, match="CUDA"):                     # everything fits: the device is what is left to refuse
         sgq.linear_w8a8(torch.zeros(3, 32), q, torch.zeros(8))
+
+
+@pytest.mark.gpu
+def test_scratch_comes_from_the_workspace_objects_own_get(sgq):
+    """A caller's workspace is asked through get(), whether it derives from Workspace and overrides it or only has it; one that
+    has nothing to give leaves the call without scratch."""
+    x, w = torch.randn(2, 256, device="cuda"), torch.randn(256, 96, device="cuda")
+    q = sgq.quantize_int4(w, 32)
+    want = sgq.quantized_matmul(x, q)
+    asked = []
+
+    class Derived(sgq.Workspace):
+        def get(self, nbytes):
+            asked.append(nbytes)
+            return super().get(nbytes)
+
+    class Duck:
+        def get(self, nbytes):
+            asked.append(nbytes)
+            return torch.empty(nbytes + 64, dtype=torch.uint8, device="cuda")
+
+    for ws in (Derived(x.device), Duck()):
+        asked.clear()
+        for _ in range(3):
+            assert torch.equal(sgq.quantized_matmul(x, q, workspace=ws), want)
+        assert asked == [sgq.linear_workspace_bytes(4, 2, 256, 96, sgq.LAYOUT_KN)] * 3
+
+    class Nothing:
+        def get(self, nbytes):
+            return None
+
+    serial = sgq.quantized_matmul(x, q, path=sgq.PATH_SIMT)
+    assert torch.equal(sgq.quantized_matmul(x, q, workspace=Nothing()), serial)
+    assert torch.equal(sgq.quantized_matmul_backward_x(want, q, workspace=Nothing()), sgq.quantized_matmul_backward_x(want, q, path=sgq.PATH_SIMT))
