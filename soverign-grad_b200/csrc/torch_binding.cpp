@@ -81,22 +81,23 @@ at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Tensor& l
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// What a QuantizedTensor holds.
+// What a QuantizedTensor holds.  Its scheme is read for INT8 only and its group for INT4 only: what a checkpoint loader left
+// in the other one does not matter.
 struct Quantized {
     at::Tensor qdata, scales;
-    int64_t scheme, group, bits, rows = 0, cols = 0, numel = 1;
+    int64_t scheme = SGQ_PER_TENSOR, group = 0, bits, rows = 0, cols = 0, numel = 1;
     size_t dims;
     Ref shape;
     explicit Quantized(PyObject* q) {
-        Ref d(PyObject_GetAttr(q, s_qdata)), s(PyObject_GetAttr(q, s_scales)), sch(PyObject_GetAttr(q, s_scheme)),
-            g(PyObject_GetAttr(q, s_group)), b(PyObject_GetAttr(q, s_bits));
+        Ref d(PyObject_GetAttr(q, s_qdata)), s(PyObject_GetAttr(q, s_scales)), b(PyObject_GetAttr(q, s_bits));
         shape.p = PyObject_GetAttr(q, s_shape);
-        if (!d || !s || !sch || !g || !b || !shape) throw PythonError();
+        if (!d || !s || !b || !shape) throw PythonError();
         qdata = as_tensor(d.p);
         scales = as_tensor(s.p);
-        scheme = as_int(sch.p);
-        group = as_int(g.p);
         bits = as_int(b.p);
+        Ref v(PyObject_GetAttr(q, bits == 4 ? s_group : s_scheme));
+        if (!v) throw PythonError();
+        (bits == 4 ? group : scheme) = as_int(v.p);
         Ref seq(PySequence_Fast(shape.p, "original_shape is a sequence"));
         if (!seq) throw PythonError();
         dims = static_cast<size_t>(PySequence_Fast_GET_SIZE(seq.p));

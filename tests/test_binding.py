@@ -76,3 +76,16 @@ def test_scratch_comes_from_the_workspace_objects_own_get(sgq):
     serial = sgq.quantized_matmul(x, q, path=sgq.PATH_SIMT)
     assert torch.equal(sgq.quantized_matmul(x, q, workspace=Nothing()), serial)
     assert torch.equal(sgq.quantized_matmul_backward_x(want, q, workspace=Nothing()), sgq.quantized_matmul_backward_x(want, q, path=sgq.PATH_SIMT))
+
+
+@pytest.mark.gpu
+def test_fields_that_a_bit_width_does_not_use_are_not_read(sgq):
+    """INT4 has no scheme and INT8 no group: what a checkpoint loader left there does not matter."""
+    x, w = torch.randn(2, 256, device="cuda"), torch.randn(256, 96, device="cuda")
+    q4, q8 = sgq.quantize_int4(w, 32), sgq.quantize_int8(w)
+    bare4 = sgq.QuantizedTensor(q4.qdata, q4.scales, None, (256, 96), 32, 4)
+    bare8 = sgq.QuantizedTensor(q8.qdata, q8.scales, sgq.PER_ROW, (256, 96), None, 8)
+    for q, bare, deq in ((q4, bare4, sgq.dequantize_int4), (q8, bare8, sgq.dequantize_int8)):
+        assert torch.equal(sgq.quantized_matmul(x, bare), sgq.quantized_matmul(x, q))
+        assert torch.equal(deq(bare), deq(q))
+    assert torch.equal(sgq.linear_w8a8(x[:, :96].contiguous(), bare8), sgq.linear_w8a8(x[:, :96].contiguous(), q8))
