@@ -643,6 +643,7 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (lane == 0) mbar_arrive(xempty);
         }
     }
+    settle_unless(alive);
 }
 
 struct Plan {

@@ -401,6 +401,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // no second barrier: the next block writes the other slot, and nobody reaches the block after
         // that before every thread has passed the next barrier, i.e. finished reading this slot
     }
+    settle_unless(alive);
 }
 
 struct Plan {

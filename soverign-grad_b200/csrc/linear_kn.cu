@@ -350,17 +350,15 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 woff[i] = (nb >> 2) * (kStageK * 128) + r * 128 + (((2 * (nb & 3) + (g >> 2)) ^ (r & 7)) << 4) + (g & 3) * 4;
             }
         }
-        bool alive = true;
         int slot = 0;
         uint32_t ph = 0;
         for (int s = s0; s < s1; ++s) {
-            if (alive && !mbar_wait(&full[slot], ph)) {
+            // One answer for the warp.  A warp that gives up hands nothing back, so the producer requests no more, and what it
+            // did request is as old as this wait when the CTA ends.
+            const bool ready = mbar_wait(&full[slot], ph) && (BITS == 4 || mbar_wait(&frag_full[(s - s0) & 1], ((s - s0) >> 1) & 1u));
+            if (!__all_sync(0xffffffffu, ready)) {
                 if (lane == 0) report(kDevErrFullWait, s);
-                alive = false;
-            }
-            if (BITS == 8 && alive && !mbar_wait(&frag_full[(s - s0) & 1], ((s - s0) >> 1) & 1u)) {
-                if (lane == 0) report(kDevErrFullWait, 0x400000u | s);
-                alive = false;
+                break;
             }
             const uint8_t* sw = smem + slot * C::kStage;
             const uint8_t* sx = sw + C::kW;

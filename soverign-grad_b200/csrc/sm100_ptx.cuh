@@ -92,10 +92,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait.  A first try without a time hint: it returns in 25 cycles when the phase is complete, the hinted form takes
-// 100 (measured), and in a running pipeline most waits find their phase complete.  After that every try_wait may suspend the warp for up to kWaitSliceNs (it wakes as soon as the
-// phase completes), so a waiting warp costs a handful of instructions per slice instead of spinning
-// through the issue slots the working warps need; after kWaitSlices slices (about 0.7 s) it gives
-// up.  false = gave up.
+// 100 (measured), and in a running pipeline most waits find their phase complete.  After that every try_wait may suspend
+// the warp for up to kWaitSliceNs (it wakes as soon as the phase completes), so a waiting warp costs a handful of
+// instructions per slice instead of spinning through the issue slots the working warps need; after kWaitSlices slices
+// (about 0.7 s) it gives up.  false = gave up.
 constexpr uint32_t kWaitSliceNs = 20000;
 constexpr uint32_t kWaitSlices = 1u << 15;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
@@ -119,6 +119,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitSliceNs), "r"(kWaitSlices)
         : "memory");
     return ok != 0;
+}
+
+// Called at the end of a role whose wait may have run out: keeps the CTA, and with it the shared memory that copies in flight
+// write, for a millisecond more.  A consumer that gave up goes on handing slots back, so the producer requests the rest of its
+// work within microseconds and nobody waits for it; without this the CTA could end under those copies.
+__device__ __forceinline__ void settle_unless(bool alive) {
+    for (int i = 0; i < 1000 && !alive; ++i) __nanosleep(1000);
 }
 
 // 2-D TMA tile load, global -> this CTA's shared memory, completion on an mbarrier.
