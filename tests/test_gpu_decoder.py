@@ -376,10 +376,10 @@ def test_greedy_decode_at_benchmark_dimensions(sgq, nl, port, prefill, tol):
     torch.cuda.empty_cache()
 
 
-def test_overlapped_launches_agree_with_serial_ones(sgq, nl, port):
-    """Programmatic dependent launch on (the default of the model) and off: the same bits; with the
-    two-CTAs-per-SM form of the decode kernel (mode 2): same tokens, logits equal up to fp32 summation
-    order (that form adds its partial sums in a different order)."""
+def test_overlap_modes_agree(sgq, nl, port):
+    """Weights fetched before older kernels are complete (mode 1, the default of the model) and only behind them (mode 0): the
+    same bits; with the two-CTAs-per-SM form of the decode kernel (mode 2): same tokens, logits equal up to fp32 summation
+    order (that form adds its partial sums in a different order).  What the kernels compute is compared with the port above."""
     _, _, tok_on, log_on, _ = tiny_model(nl, port, prompt_len=9, n_new=6, prefill_path=sgq.PATH_SIMT, overlap=1)
     _, _, tok_off, log_off, _ = tiny_model(nl, port, prompt_len=9, n_new=6, prefill_path=sgq.PATH_SIMT, overlap=0)
     _, _, tok_two, log_two, _ = tiny_model(nl, port, prompt_len=9, n_new=6, prefill_path=sgq.PATH_SIMT, overlap=2)
@@ -393,8 +393,8 @@ def test_overlapped_launches_agree_with_serial_ones(sgq, nl, port):
 
 @pytest.mark.parametrize("M,K", [(1, 4096), (4, 4096), (8, 2048), (16, 2048), (8, 5632), (3, 256)])
 def test_overlap_switch_on_back_to_back_linears(sgq, M, K):
-    """A chain of decode forwards whose inputs are the previous outputs, with and without overlap
-    (overlapped launches use the two-CTAs-per-SM form of the decode kernel)."""
+    """A chain of decode forwards whose inputs are the previous outputs: waited for one by one, then back to back in every mode
+    (mode 2 uses the two-CTAs-per-SM form of the decode kernel)."""
     g = torch.Generator(device="cuda").manual_seed(11 + M)
     qs = [sgq.quantize_int4(torch.randn(K, K, device="cuda", generator=g) * (1.5 / K ** 0.5), 32) for _ in range(4)]
     x0 = torch.randn(M, K, device="cuda", generator=g)
@@ -407,6 +407,8 @@ def test_overlap_switch_on_back_to_back_linears(sgq, M, K):
                 if keep is not None:
                     keep.append(x)
                 x = sgq.quantized_matmul(x, q, None, layout=sgq.LAYOUT_NK, path=sgq.PATH_GEMV, workspace=ws)
+                if keep is not None:
+                    torch.cuda.synchronize()                              # the serial run: nothing overlaps anything
         return x
 
     prev = sgq.set_stream_overlap(False)
@@ -414,6 +416,7 @@ def test_overlap_switch_on_back_to_back_linears(sgq, M, K):
         inputs = []
         want = chain(inputs)
         outputs = inputs[1:] + [want]
+        assert torch.equal(chain(), want)                                 # mode 0: launched back to back, weights behind the wait
         sgq.set_stream_overlap(1)
         assert torch.equal(chain(), want)                                 # overlapped launches alone change no bit
         sgq.set_stream_overlap(2)                                         # ... the two-CTAs-per-SM form changes the summation order

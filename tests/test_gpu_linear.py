@@ -146,6 +146,33 @@ def test_decode_int8_kernel_against_port(sgq, port, M, K, N):
     assert err.value.status == 5
 
 
+# (N / 16 tiles over 148 SMs: up to two tiles per CTA are worked on in blocks of two, from three on in blocks of four)
+TILE_BLOCKS_I8 = [(1, 1024, 2601), (16, 4224, 2601), (4, 8192, 4735), (2, 1152, 4999), (5, 2176, 5003), (7, 128, 4737), (9, 1664, 7217),
+                  (12, 640, 9491), (15, 1280, 14001), (3, 1408, 11008)]
+
+
+@pytest.mark.parametrize("M,K,N", TILE_BLOCKS_I8)
+def test_decode_int8_blocks_of_tiles(sgq, M, K, N):
+    """The INT8 decode kernel's blocks of two and of four tiles: a last tile that is not whole, blocks that are not, a last stage
+    of one to seven steps, every layout of the digit sets, scales per row and per tensor, and rows whose outliers flag the low
+    digits, all outputs against an exact model of the kernel's arithmetic (on the GPU in float64) and the fp32 contract."""
+    x = heavy_tailed_rows(M * 7 + N, M, K, 300.0, 3) * np.random.default_rng(N).uniform(0.1, 30.0, (M, 1)).astype(np.float32)
+    gen = torch.Generator(device="cuda").manual_seed(M + K + N)
+    w = torch.randn(N, K, device="cuda", generator=gen) * 0.02
+    b = torch.randn(N, device="cuda", generator=gen) * 0.1
+    held = dev(block_fixed_point(x, 128))
+    ws = sgq.Workspace(torch.device("cuda"))
+    for scheme in (cases.PER_TENSOR, cases.PER_ROW):
+        q = sgq.quantize_int8(w, scheme)
+        for bias in (b, None):
+            y = sgq.quantized_matmul(dev(x), q, bias, layout=cases.LAYOUT_NK, path=sgq.PATH_GEMV, workspace=ws).cpu().numpy()
+            check_status(sgq)
+            deq, add = q.qdata.double() * q.scales.double().view(-1, 1), 0.0 if bias is None else bias.double()
+            model, want = (held @ deq.t() + add).cpu().numpy(), (dev(x).double() @ deq.t() + add).cpu().numpy()
+            assert rel_err(y, model) <= (2e-6 if M <= 2 else 1e-4), ("layout/pipeline error, not rounding", scheme, rel_err(y, model))
+            assert rel_err(y, want) <= TOL_FP32
+
+
 def test_decode_kernel_rejects_what_it_cannot_run(sgq):
     w = torch.randn(64, 96, device="cuda")       # K = 96 is not a multiple of 256
     q = sgq.quantize_int4(w, 32)
@@ -276,35 +303,59 @@ def test_tc_bf16_against_port(sgq, port, M, K, N):
         assert rel_err(y, want) <= (TOL_BF16 if K >= 1024 else 8e-2), rel_err(y, want)
 
 
+@pytest.mark.parametrize("layout", [cases.LAYOUT_NK, cases.LAYOUT_KN])
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("M,K,N", [(2048, 4096, 11008), (512, 2048, 4096), (200, 192, 1000), (64, 64, 40), (300, 384, 520),
-                                   (130, 256, 70), (1100, 5632, 2048)])
-def test_tc_bf16_gemm_that_starts_during_the_expansion(sgq, bits, M, K, N):
-    """With overlapped launches the GEMM starts while the weight is still being expanded into the scratch and waits
-    on per-part counters.  Forwards with DIFFERENT weights through the SAME scratch, back to back, must give the
-    bits of the serial launches: a tile read before its rows were rewritten would show the previous weight."""
+@pytest.mark.parametrize("M,K,N", [(256, 4096, 28672), (2048, 4096, 11008), (512, 2048, 4096), (1100, 5632, 2048), (130, 256, 96),
+                                   (300, 384, 544), (200, 192, 1024), (64, 64, 64)])
+def test_tc_bf16_gemm_that_starts_during_the_expansion(sgq, bits, layout, M, K, N):
+    """The GEMM starts while the weight is still being expanded into the scratch, slice of K by slice of K (eight slices for the
+    first shape, then four, two for K = 384, one for K of 192 and 64), and waits on a counter per slice.  Expected: one forward
+    per weight in a scratch of its own that holds NaN, waited for, and checked against a float64 product of the operands as the
+    path rounds them.  Forwards with DIFFERENT weights through the SAME scratch, back to back, must give those bits: a tile
+    read before its slice was rewritten would show the weight, or the activations, of the forward before."""
+    n = N if layout == cases.LAYOUT_KN else N - 26                 # [N,K] may be ragged
     g = torch.Generator(device="cuda").manual_seed(M + N + bits)
-    x = torch.randn(M, K, device="cuda", generator=g)
+    xs = [torch.randn(M, K, device="cuda", generator=g) for _ in range(2)]
     ws = []
     for i in range(4):
-        w = torch.randn(N, K, device="cuda", generator=g) * (0.02 * (i + 1))
+        w = torch.randn((K, n) if layout == cases.LAYOUT_KN else (n, K), device="cuda", generator=g) * (0.02 * (i + 1))
         ws.append(sgq.quantize_int4(w, 32) if bits == 4 else sgq.quantize_int8(w, cases.PER_ROW))
-    space = sgq.Workspace(torch.device("cuda"))
-    outs = {}
+        del w
+    forward = dict(layout=layout, path=sgq.PATH_TC_BF16)
+    need = sgq.linear_workspace_bytes(bits, M, K, n, layout, sgq.PATH_TC_BF16)
+    rows = torch.unique(torch.linspace(0, M - 1, 24, device="cuda").long())
+    cols = torch.unique(torch.linspace(0, n - 1, 48, device="cuda").long())
+    want = []
+    for i in range(8):
+        fresh = sgq.Workspace(torch.device("cuda"))
+        fresh.get(need).fill_(0xFF)                                # bf16 NaN in both operands
+        x, q = xs[i % 2], ws[i % 4]
+        want.append(sgq.quantized_matmul(x, q, None, workspace=fresh, **forward))
+        torch.cuda.synchronize()
+        check_status(sgq)
+        real = (sgq.dequantize_int4 if bits == 4 else sgq.dequantize_int8)(q)
+        real = real[:, cols] if layout == cases.LAYOUT_KN else real[cols].t()
+        if not (bits == 8 and layout == cases.LAYOUT_NK):          # INT8 [N,K]: exact codes, the scale in fp32 afterwards
+            real = real.bfloat16()
+        xr, wr = x[rows].bfloat16().double(), real.double()
+        got = want[-1][rows][:, cols].double()
+        # exact products, K fp32 sums of them and the epilogue's rounding, 2^-23 of the running magnitude each
+        assert bool(((got - xr @ wr).abs() <= (xr.abs() @ wr.abs()) * (K + 4) * 2.0 ** -23).all())
+        assert norm_err(got.cpu().numpy(), (xr @ wr).cpu().numpy()) <= 1e-4     # (a slice in a wrong place is an error of its size)
+    shared = sgq.Workspace(torch.device("cuda"))
     for mode in (0, 1):
         prev = sgq.set_stream_overlap(mode)
         try:
-            ys = [torch.empty(M, N, device="cuda") for _ in range(12)]
+            ys = [torch.empty(M, n, device="cuda") for _ in range(16)]
             for i, y in enumerate(ys):
-                sgq.quantized_matmul(x, ws[i % 4], None, layout=cases.LAYOUT_NK, path=sgq.PATH_TC_BF16, out=y, workspace=space)
+                sgq.quantized_matmul(xs[i % 2], ws[i % 4], None, out=y, workspace=shared, **forward)
             torch.cuda.synchronize()
-            outs[mode] = ys
         finally:
             sgq.set_stream_overlap(prev)
-    check_status(sgq)
-    for a, b in zip(outs[0], outs[1]):
-        assert torch.equal(a, b)
-    assert not torch.equal(outs[1][0], outs[1][1])
+        check_status(sgq)
+        for i, y in enumerate(ys):
+            assert torch.equal(y, want[i % 8]), (mode, i)
+    assert not torch.equal(want[0], want[1])
 
 
 @pytest.mark.parametrize("M,K,N", TC_SHAPES)
@@ -340,7 +391,7 @@ KN_TC_SHAPES = [(128, 64, 256), (256, 512, 512), (100, 192, 288), (300, 1024, 28
 @pytest.mark.parametrize("M,K,N", KN_TC_SHAPES)
 def test_tc_bf16_kn_layout_against_port(sgq, port, M, K, N):
     """Weights kept in the reference module's own [in, out] layout on the tensor cores: the weight is expanded
-    to bf16 (code * scale in fp32, rounded once) and transposed in front of a GEMM whose operands both arrive by TMA."""
+    to bf16 (code * scale in fp32, rounded once) in that order, in front of a GEMM whose operands both arrive by TMA."""
     rng = np.random.default_rng(5 * M + 7 * K + 11 * N)
     x = rng.standard_normal((M, K)).astype(np.float32)
     w = cases.weight_with_outliers(M + K + N + 3, (K, N))
@@ -640,3 +691,33 @@ def test_batches_converted_in_front_match_their_blocks(sgq, M, K):
         y = sgq.quantized_matmul(x, q, None, layout=cases.LAYOUT_NK, workspace=sgq.Workspace(torch.device("cuda")), workspace_limit=limit)
         check_status(sgq)
         assert torch.equal(y, blocks)
+
+
+@pytest.mark.parametrize("layout", [cases.LAYOUT_NK, cases.LAYOUT_KN])
+@pytest.mark.parametrize("M", [1, 4, 16, 40, 128])
+def test_weights_may_be_written_just_before_the_call(sgq, M, layout):
+    """With sgq_set_stream_overlap off there is no rule for the caller: weights that the launch in front has just written (the
+    quantizers, whose kernels let the next one start early, or a copy) are the ones that the forward reads, although its
+    decode kernel requests them before its own dependency wait."""
+    K = N = 4096
+    assert sgq.set_stream_overlap(0) == 0
+    g = torch.Generator(device="cuda").manual_seed(M + layout)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    floats = [torch.randn((N, K) if layout == cases.LAYOUT_NK else (K, N), device="cuda", generator=g) * 0.02 * (i + 1) for i in range(3)]
+    ws = sgq.Workspace(torch.device("cuda"))
+    for make in (lambda w: sgq.quantize_int8(w, cases.PER_TENSOR), lambda w: sgq.quantize_int8(w, cases.PER_ROW), lambda w: sgq.quantize_int4(w, 32)):
+        made = [make(w) for w in floats]
+        torch.cuda.synchronize()
+        want = []
+        for q in made:
+            want.append(sgq.quantized_matmul(x, q, layout=layout, workspace=ws))
+            torch.cuda.synchronize()
+        held = make(floats[0])
+        for i in range(12):
+            held.qdata.copy_(made[i % 3].qdata)
+            held.scales.copy_(made[i % 3].scales)
+            copied = sgq.quantized_matmul(x, held, layout=layout, workspace=ws)
+            # quantized into a buffer that still holds another weight's codes (the allocator hands it out again)
+            quantized = sgq.quantized_matmul(x, make(floats[i % 3]), layout=layout, workspace=ws)
+            assert torch.equal(copied, want[i % 3]) and torch.equal(quantized, want[i % 3]), i
+    check_status(sgq)
