@@ -106,21 +106,6 @@ __device__ __forceinline__ void mma_s8s8_16832_magic(int (&d)[4], const uint32_t
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(kMagicBits));
 }
 
-// N consecutive floats (16-byte aligned for N = 4, 8-byte for N = 2) with the widest load that fits.
-template <int N>
-__device__ __forceinline__ void load_scales(float (&v)[N], const float* p) {
-    if constexpr (N == 4) {
-        const float4 q = *reinterpret_cast<const float4*>(p);
-        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    } else if constexpr (N == 2) {
-        const float2 q = *reinterpret_cast<const float2*>(p);
-        v[0] = q.x; v[1] = q.y;
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) v[i] = p[i];
-    }
-}
-
 // Four 8x8 matrices of 16-byte rows: lane l supplies the address of row (l & 7) of matrix (l >> 3);
 // lane (g, t) receives word t of row g of every matrix.
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_addr) {

@@ -102,11 +102,6 @@ __device__ __forceinline__ void kn_cp_async_16(uint32_t dst, const void* src, in
 __device__ __forceinline__ void kn_cp_async_4(uint32_t dst, const void* src, int bytes) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -427,7 +422,7 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 for (int j = 0; j < T; ++j)
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        mma_bf16(acc[i][T <= 2 ? j : 2 * (j / 3) + (j % 3 ? 1 : 0)], a[i], frag[j].x, frag[j].y);
+                        mma_bf16_16816(acc[i][T <= 2 ? j : 2 * (j / 3) + (j % 3 ? 1 : 0)], a[i], frag[j].x, frag[j].y);
             }
             uint32_t fold = 0;
 #pragma unroll
