@@ -489,6 +489,10 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         const float* sg = sxs + (static_cast<size_t>(step) * 8 * 4 + t) * (2 * NM);      // this lane's group scales
                         const uint8_t* fg = flg + static_cast<size_t>(step) * 8 * 16;
                         constexpr int BG = NM <= 2 ? 4 : 2;              // 32-k groups whose MMAs are in flight together
+                        // Low digits: only where a row of the set flagged the group (one value dominating it: rare in a normalised
+                        // row, common behind a gate).  One vote reads the flags of the step's eight groups (a lane per four rows):
+                        // bit 4i + 2l or the next is set where set l of group i is flagged, the same in every lane.
+                        const uint32_t flagged = NL > 0 ? __ballot_sync(0xffffffffu, reinterpret_cast<const uint32_t*>(fg)[lane] != 0u) : 0u;
 #pragma unroll
                         for (int hb = 0; hb < 8 / BG; ++hb) {
                             const int hh = (hb * BG) >> 2;               // which half of the step: 16-byte unit of the scales
@@ -497,21 +501,19 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                             uint32_t wv[BG / 2][4];                      // [pair of groups]{rows 0-7, rows 8-15} x 2
 #pragma unroll
                             for (int pq = 0; pq < BG / 2; ++pq) ldmatrix_x4(wv[pq], wbox + lm_off[(hb * BG) / 2 + pq]);
-                            // Low digits: only where a row of the set flagged the group (one value dominating it: rare in a
-                            // normalised row, common behind a gate).  They lie in global memory, so the fragments of all
-                            // flagged groups are requested together, before the main MMAs; fetched one by one where they
-                            // are used they cost an L2 round trip per group.
+                            // They lie in global memory, so the fragments of all flagged groups are requested together, before the
+                            // main MMAs; fetched one by one where they are used they cost an L2 round trip per group (generation,
+                            // batch 8: 135.1 ms, 130.0 so).  A flag test per group in front of the MMAs, in place of the vote, cost
+                            // rows without flagged groups more than it gave (8 rows, 4096 x 11008: 13.9 us, 12.4 so).
                             uint2 lowq[BG][NL > 0 ? NL : 1];
                             float2 lowsc[BG][NL > 0 ? NL : 1];
-                            uint32_t flagged = 0;                        // bit i * NL + l, the same in every lane of the warp
+                            if (NL > 0 && ((flagged >> (4 * hb * BG)) & ((1u << (4 * BG)) - 1u)) != 0u) {
 #pragma unroll
-                            for (int i = 0; i < BG; ++i) {
+                                for (int i = 0; i < BG; ++i) {
 #pragma unroll
-                                for (int l = 0; l < NL; ++l) {
-                                    const uint2 fl = *reinterpret_cast<const uint2*>(fg + (hb * BG + i) * 16 + l * 8);
-                                    if ((fl.x | fl.y) != 0u) {
+                                    for (int l = 0; l < NL; ++l) {
+                                        if (((flagged >> (4 * (hb * BG + i) + 2 * l)) & 3u) == 0u) continue;
                                         const size_t grp = static_cast<size_t>(step) * 8 + hb * BG + i;       // group within the phase
-                                        flagged |= 1u << (i * NL + l);
                                         lowq[i][l] = *reinterpret_cast<const uint2*>(lowd + plane_offset(grp, NL, l, lane));
                                         lowsc[i][l] = *reinterpret_cast<const float2*>(lows + ((grp * 4 + t) * NL + l) * 2);
                                     }
@@ -568,7 +570,7 @@ gemv_int4_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                                 }
 #pragma unroll
                                 for (int l = 0; l < NL; ++l) {
-                                    if ((flagged >> (i * NL + l)) & 1u) {
+                                    if (((flagged >> (4 * (hb * BG + i) + 2 * l)) & 3u) != 0u) {
                                         const uint2 q = lowq[i][l];
                                         const float2 sl = lowsc[i][l];
                                         int dl[4];
