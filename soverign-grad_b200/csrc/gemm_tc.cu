@@ -606,7 +606,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     report(kDevErrEmptyWait, 0x800000u);
                     alive = false;
                 }
-            settle_unless(alive);
+            for (int i = 0; i < 1000 && !alive; ++i) __nanosleep(1000);
         }
         __syncwarp();
     } else if (warp == 1) {

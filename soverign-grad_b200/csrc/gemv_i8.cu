@@ -257,7 +257,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const uint8_t* low_digits = planes + piece_bytes(groups_total, NM, NL);
     const float* low_scales = reinterpret_cast<const float*>(low_digits + static_cast<size_t>(groups_total) * NL * 256);
 
-    bool alive = true;
+    bool alive = true;                              // false after a wait ran out: nothing is handed back, the producer stops
     int st = 0;
     uint32_t ph = 0;
     for (int blk = 0; blk < nblocks; ++blk) {
@@ -331,7 +331,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
             for (int s = 0; s < NM + NL; ++s) fold ^= __float_as_uint(total[s][0]) ^ __float_as_uint(total[s][3]);
             const uint32_t landed = loads_landed(fold);
-            if (lane == 0) mbar_arrive_after(&empty[st], landed);
+            if (lane == 0 && alive) mbar_arrive_after(&empty[st], landed);
             if (++st == nstages) { st = 0; ph ^= 1u; }
         }
 
@@ -379,7 +379,6 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // no second barrier: the next block writes the other slot, and nobody reaches the block after
         // that before every thread has passed the next barrier, i.e. finished reading this slot
     }
-    settle_unless(alive);
 }
 
 struct Plan {

@@ -121,13 +121,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Called at the end of a role whose wait may have run out: keeps the CTA, and with it the shared memory that copies in flight
-// write, for a millisecond more.  A consumer that gave up goes on handing slots back, so the producer requests the rest of its
-// work within microseconds and nobody waits for it; without this the CTA could end under those copies.
-__device__ __forceinline__ void settle_unless(bool alive) {
-    for (int i = 0; i < 1000 && !alive; ++i) __nanosleep(1000);
-}
-
 // 2-D TMA tile load, global -> this CTA's shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t x,
                                             int32_t y) {
