@@ -31,7 +31,7 @@
 // 1e-3 contract.  The split holds away from the ends of the exponent range only: the remainders of an Inf, and of a finite
 // factor above bf16's largest value, are Inf - Inf, and those of a factor below about 2^-110 end under bf16's smallest.  The
 // first makes every output of its row NaN, the second leaves outputs near zero, so the epilogue recognises both by the sum
-// itself and forms such an output again as the plain chain of fp32 multiply-adds (kn_chain4): +-Inf and NaN per output as
+// itself and, behind its last store, forms such an output again as the plain chain of fp32 multiply-adds (kn_chain4): +-Inf and NaN per output as
 // in the reference, and no loss for vanishing rows.
 #include "sgq_common.cuh"
 #include "sm100_ptx.cuh"
@@ -82,6 +82,7 @@ struct KnMmaParams {
     const float* scales;
     int scale_mode;          // 0: INT4 groups, 1: one per k, 2: one
     int64_t group;           // INT4: a multiple of 32 that divides N
+    int64_t per_row;         // INT4: scales per k (N / group; a division per stage in the producer cost 4096 x 5792 10 %)
     int group_shift;         // log2(group / 32), or -1
     int pitch;               // INT4: scales per k in a stage (groups that a CTA's features span)
     int vec_scales;          // INT4: a stage's scales can be copied 16 bytes at a time
@@ -92,7 +93,7 @@ struct KnMmaParams {
     int M;
     int64_t K, N;
     int early;               // weights may be requested before the dependency wait (overlapped launches)
-    const float* x;          // operands by address, for kn_chain4
+    const float* x;          // the operands by address, for kn_chain4
     const uint8_t* wq;
 };
 
@@ -123,27 +124,28 @@ __device__ __forceinline__ void split3(float p0, float p1, uint32_t (&part)[3]) 
     }
 }
 
-// Whether a sum (without the bias) may come from factors that the split does not hold exactly: not finite, or below 2^-90 and
+// Whether one of four sums (without the bias) may come from factors that the split does not hold exactly: not finite, or below 2^-90 and
 // not zero.  (Factors below 2^-110, or 2^-117 where remainders under 2^-126 count as zero, are wrong by at most 2^-126: 2^13
 // of them times a code of 8 are 2^-110, a millionth of the smallest sum that passes.  A row of zeros is exact.)
-__device__ __forceinline__ bool kn_sum_suspect(float v) {
-    const float a = fabsf(v);
-    return !(a >= 8.07793567e-28f && a <= 3.402823466e+38f) && a != 0.0f;      // true for NaN
+__device__ __forceinline__ bool kn_sums_suspect(const float4& v) {
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float a = fabsf(j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w);
+        ok = ok && ((a >= 8.07793567e-28f && a <= 3.402823466e+38f) || a == 0.0f);
+    }
+    return !ok;
 }
 
-// Outputs (m, n .. n + 3) as one chain of fp32 multiply-adds each, in ascending k.  A call of its own (not inlined): it runs for
-// rows at the ends of the exponent range only, and its registers are not the kernel's.
+// Four neighbouring outputs as one chain of fp32 multiply-adds each, in ascending k; x: the row of activations, w and s: the
+// codes and the scale at k = 0.  A call of its own (not inlined) with its arguments by value: it runs for rows at the ends of the
+// exponent range only, its registers are not the kernel's, and the parameter block keeps no address.
 template <int BITS>
-__device__ __noinline__ float4 kn_chain4(const KnMmaParams& p, int m, int64_t n) {
+__device__ __noinline__ float4 kn_chain4(const float* x, const uint8_t* w, const float* s, int64_t K, int64_t row_bytes, int64_t scale_step) {
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const float* x = p.x + static_cast<int64_t>(m) * p.K;
-    const int64_t row_bytes = BITS == 4 ? p.N / 2 : p.N;
-    const uint8_t* w = p.wq + (BITS == 4 ? n / 2 : n);
-    const int64_t per_row = BITS == 4 ? p.N / p.group : 1;
-    const float* s = p.scales + (BITS == 4 ? n / p.group : 0);          // a group holds whole runs of 32 features
 #pragma unroll 4
-    for (int64_t k = 0; k < p.K; ++k) {
-        const float f = x[k] * (p.scale_mode == 2 ? s[0] : s[k * per_row]);
+    for (int64_t k = 0; k < K; ++k) {
+        const float f = x[k] * s[k * scale_step];
         const uint32_t c = BITS == 4 ? *reinterpret_cast<const uint16_t*>(w + k * row_bytes) : *reinterpret_cast<const uint32_t*>(w + k * row_bytes);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -154,7 +156,7 @@ __device__ __noinline__ float4 kn_chain4(const KnMmaParams& p, int m, int64_t n)
 
 template <int BITS, int T, int NBW>
 __global__ void __launch_bounds__(kMmaThreads, 2)
-kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ KnMmaParams p) {
+kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const KnMmaParams p) {
     using C = KnCfg<BITS, T, NBW>;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -262,7 +264,7 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             const uint32_t dst = smem_u32(sx + 2 * C::kXBox);
             const int64_t k0 = static_cast<int64_t>(s) * kStageK;
             if (BITS == 4 && p.group_shift >= 0) {
-                const int64_t per_row = p.N / p.group, g0 = (n0 / 32) >> p.group_shift;
+                const int64_t per_row = p.per_row, g0 = (n0 / 32) >> p.group_shift;
                 if (p.vec_scales) {
                     const int quads = p.pitch / 4;                              // 1 or 2
                     for (int c = lane; c < kStageK * quads; c += 32) {
@@ -280,7 +282,7 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                     }
                 }
             } else if (BITS == 4) {
-                const int64_t per_row = p.N / p.group;
+                const int64_t per_row = p.per_row;
                 for (int q = 0; q < kStageK * NBW / 32; ++q) {
                     const int e = lane + 32 * q, row = e / NBW, w = e % NBW;
                     const int64_t k = k0 + row, n = n0 + 32 * w;
@@ -462,8 +464,19 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         }
     }
     cluster.sync();                                          // every CTA's sums are in its shared memory
-    const int quads = C::kFeatures / 4;
-    for (int e = rank * kMmaThreads + threadIdx.x; e < p.M * quads; e += ranks * kMmaThreads) {
+    const int quads = C::kFeatures / 4, step = ranks * kMmaThreads;
+    uint32_t suspect = 0;                                    // bit per quad of this thread (at most 16 * 64 / 320 = 4)
+    auto store = [&](float4 v, int m, int64_t n) {
+        if (p.bias) { v.x += p.bias[n]; v.y += p.bias[n + 1]; v.z += p.bias[n + 2]; v.w += p.bias[n + 3]; }
+        float* dst = p.y + static_cast<int64_t>(m) * p.ldy + n;
+        if (p.vec_y) {
+            *reinterpret_cast<float4*>(dst) = v;
+        } else {
+            dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
+        }
+    };
+    uint32_t bit = 1;
+    for (int e = rank * kMmaThreads + threadIdx.x; e < p.M * quads; e += step, bit <<= 1) {
         const int m = e / quads, c = (e - m * quads) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int r = 0; r < ranks; ++r) {
@@ -474,19 +487,21 @@ kn_mma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
             }
         }
-        const int64_t n = n0 + c;
-        if (n < p.N) {                                       // N % 4 == 0
-            if (kn_sum_suspect(v.x) || kn_sum_suspect(v.y) || kn_sum_suspect(v.z) || kn_sum_suspect(v.w)) v = kn_chain4<BITS>(p, m, n);
-            if (p.bias) { v.x += p.bias[n]; v.y += p.bias[n + 1]; v.z += p.bias[n + 2]; v.w += p.bias[n + 3]; }
-            float* dst = p.y + static_cast<int64_t>(m) * p.ldy + n;
-            if (p.vec_y) {
-                *reinterpret_cast<float4*>(dst) = v;
-            } else {
-                dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
-            }
+        if (n0 + c < p.N) {                                  // N % 4 == 0
+            store(v, m, n0 + c);
+            if (kn_sums_suspect(v)) suspect |= bit;
         }
     }
     cluster.sync();                                          // shared memory stays until the others have read it
+    if (suspect != 0) {
+        for (int e = rank * kMmaThreads + threadIdx.x; suspect != 0; e += step, suspect >>= 1) {
+            if ((suspect & 1u) == 0) continue;
+            const int m = e / quads, c = (e - m * quads) * 4;
+            const int64_t n = n0 + c;
+            store(kn_chain4<BITS>(p.x + static_cast<int64_t>(m) * p.K, p.wq + (BITS == 4 ? n / 2 : n), p.scales + (BITS == 4 ? n / p.group : 0), p.K,
+                                  BITS == 4 ? p.N / 2 : p.N, BITS == 4 ? p.per_row : (p.scale_mode == 1 ? 1 : 0)), m, n);
+        }
+    }
 }
 
 // Features per CTA (256 or 128) and slices of K (the cluster size): the split with the shortest longest CTA, in stages of 64 k
@@ -523,6 +538,7 @@ int launch_mma(const LinearArgs& a, int slices) {
     p.scales = a.scales;
     p.scale_mode = BITS == 4 ? 0 : (a.scheme == SGQ_PER_ROW ? 1 : 2);
     p.group = a.group;
+    p.per_row = BITS == 4 ? a.N / a.group : 1;
     p.group_shift = -1;
     p.pitch = NBW;
     if (BITS == 4) {
