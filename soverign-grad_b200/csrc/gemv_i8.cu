@@ -257,7 +257,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const uint8_t* low_digits = planes + piece_bytes(groups_total, NM, NL);
     const float* low_scales = reinterpret_cast<const float*>(low_digits + static_cast<size_t>(groups_total) * NL * 256);
 
-    bool alive = true;                              // false after a wait ran out: nothing is handed back, the producer stops
+    bool alive = true;                              // false after a wait ran out: skip the math, keep the barriers balanced
     int st = 0;
     uint32_t ph = 0;
     for (int blk = 0; blk < nblocks; ++blk) {
@@ -331,7 +331,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
             for (int s = 0; s < NM + NL; ++s) fold ^= __float_as_uint(total[s][0]) ^ __float_as_uint(total[s][3]);
             const uint32_t landed = loads_landed(fold);
-            if (lane == 0 && alive) mbar_arrive_after(&empty[st], landed);
+            if (lane == 0) mbar_arrive_after(&empty[st], landed);
             if (++st == nstages) { st = 0; ph ^= 1u; }
         }
 
@@ -379,6 +379,9 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // no second barrier: the next block writes the other slot, and nobody reaches the block after
         // that before every thread has passed the next barrier, i.e. finished reading this slot
     }
+    // After a wait that ran out the producer may just have requested the rest: a millisecond for the copies in flight, as the
+    // CTA must not end under them.  (Not handing slots back instead costs 16 rows of 8192 x 28672 1 %.)
+    for (int i = 0; i < 1000 && !alive; ++i) __nanosleep(1000);
 }
 
 struct Plan {

@@ -124,17 +124,17 @@ __device__ __forceinline__ void split3(float p0, float p1, uint32_t (&part)[3]) 
     }
 }
 
-// Whether one of four sums (without the bias) may come from factors that the split does not hold exactly: not finite, or below 2^-90 and
-// not zero.  (Factors below 2^-110, or 2^-117 where remainders under 2^-126 count as zero, are wrong by at most 2^-126: 2^13
+// Whether one of four sums (without the bias) may come from factors that the split does not hold exactly: not finite, or
+// below 2^-90 and not zero.  (Factors below 2^-110, or 2^-117 where remainders under 2^-126 count as zero, are wrong by at most 2^-126: 2^13
 // of them times a code of 8 are 2^-110, a millionth of the smallest sum that passes.  A row of zeros is exact.)
 __device__ __forceinline__ bool kn_sums_suspect(const float4& v) {
-    bool ok = true;
+    constexpr uint32_t kLow = 0x12800000u, kHigh = 0x7F7FFFFFu;          // 2^-90 and the largest finite value, as bits
+    const uint32_t a[4] = {__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu, __float_as_uint(v.z) & 0x7FFFFFFFu,
+                           __float_as_uint(v.w) & 0x7FFFFFFFu};
+    uint32_t far = 0;                                        // an unsigned difference is one compare for both ends
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float a = fabsf(j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w);
-        ok = ok && ((a >= 8.07793567e-28f && a <= 3.402823466e+38f) || a == 0.0f);
-    }
-    return !ok;
+    for (int j = 0; j < 4; ++j) far |= (a[j] - kLow > kHigh - kLow && a[j] != 0u) ? 1u : 0u;
+    return far != 0u;
 }
 
 // Four neighbouring outputs as one chain of fp32 multiply-adds each, in ascending k; x: the row of activations, w and s: the
