@@ -351,7 +351,7 @@ def extras(torch, sgq, peaks, copies_w, only=None, eager=False):
         return {"ms": ms, "tflops": tf, "frac_of_measured_bf16_burst": tf / peaks["bf16_tflops"],
                 "frac_of_nominal_bf16_2250": tf / 2250.0, "path": sgq.PATH_NAMES[path],
                 "includes": "activation conversion/quantization kernel + GEMM"
-                            + (" + per-forward expansion of the [K,N] weight to bf16 [N,K]" if layout == sgq.LAYOUT_KN else "")}
+                            + (" + per-forward expansion of the [K,N] weight to bf16" if layout == sgq.LAYOUT_KN else "")}
 
     def int8_tensor_peak():
         # Denominator for the W8A8 lines: the vendor library's int8 x int8 -> int32 GEMM (cuBLASLt through
@@ -875,7 +875,7 @@ def run_ours(args):
                    "path": sgq.PATH_NAMES[path], "bytes_per_launch": bytes_per_launch,
                    "launch": "one CUDA graph replay per step" if use_graph else "eager launches",
                    "stream_overlap": (f"mode {args.overlap_mode}: programmatic dependent launch, a forward's first weight tiles are "
-                                      "fetched while the previous forward finishes") if not args.no_overlap else "off"},
+                                      "fetched while the previous forward finishes") if not args.no_overlap else "mode 0"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": (achieved / peaks["hbm_gbs"]) if achieved else None,
                      "traffic": args.traffic if args.traffic is not None else ncu_traffic("gemv_int4_nk_kernel", M) if world == 1 else None,
@@ -917,9 +917,9 @@ def main():
     ap.add_argument("--no-extras", action="store_true")
     ap.add_argument("--no-graph", action="store_true", help="launch eagerly instead of replaying a CUDA graph")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--no-overlap", action="store_true", help="launch without programmatic dependent launch")
+    ap.add_argument("--no-overlap", action="store_true", help="weights are fetched only when older kernels are complete (mode 0)")
     ap.add_argument("--overlap-mode", type=int, default=1, choices=[1, 2],
-                    help="1: overlapped launches; 2: overlapped launches with the two-CTAs-per-SM form of the decode kernel")
+                    help="1: first weight tiles fetched early; 2: also the two-CTAs-per-SM form of the decode kernel")
     ap.add_argument("--nccl", action="store_true", help="N > 1: exchange output slices with an NCCL all-gather instead of peer stores")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     args = ap.parse_args()

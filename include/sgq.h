@@ -91,19 +91,20 @@ SGQ_API const char* sgq_status_string(int status);
 SGQ_API const char* sgq_last_error(void);
 SGQ_API int sgq_abi_version(void);
 
-/* Overlap of consecutive kernels in a stream (programmatic dependent launch; process-wide switch,
- * off by default, returns the previous setting; no counterpart in the reference).  With 1, every
- * kernel of this library is launched so that it may start while the kernel before it in the same
- * stream is still finishing: its set-up, and for the decode kernel the first tiles of WEIGHTS and
- * SCALES, are fetched early; activations, workspaces and outputs are touched only after the
- * earlier kernel has completed, so results are the same bits as without overlap.  With 2 the INT4
- * decode kernel additionally runs as two smaller CTAs per SM, so that the next forward's CTA can sit
- * beside the running one; that form adds its fp32 partial sums in another order (results equal to
- * fp32 rounding, bit-identical run to run) and measured no faster than 1 on B200.  The one rule
- * the switch adds: a weight, scale or bias buffer must not be the output of the kernel launched
- * immediately before the linear that reads it in the same stream (quantize, then run something
- * else or synchronise, then multiply).  It pays in launch-bound sequences: a decode step is ~130
- * kernels of 3-17 us. */
+/* When a decode kernel may fetch WEIGHTS and SCALES (process-wide switch, off by default, returns the previous
+ * setting; no counterpart in the reference).  Kernels of this library are always launched with programmatic
+ * stream serialization: one may set itself up while the kernel before it in the stream finishes, and waits
+ * for that kernel before it touches anything the kernel could have written.  That adds no rule for the caller.
+ * With 0 weights are fetched when everything older than the call is complete: behind that wait, or, where the call
+ * converts its activations in a kernel of its own, beside that kernel, which lets the decode kernel start behind its
+ * own wait only.  With 1 the first tiles of weights and scales are fetched while older kernels still run;
+ * activations, workspaces and outputs are touched only after the earlier kernel has completed, so results are
+ * the same bits.  With 2 the INT4 decode kernel additionally runs as two smaller CTAs per SM, so that the next
+ * forward's CTA can sit beside the running one; that form adds its fp32 partial sums in another order (results
+ * equal to fp32 rounding, bit-identical run to run) and measured no faster than 1 on B200.  The one rule that 1
+ * and 2 add: a weight, scale or bias buffer must not be the output of the kernel launched immediately before
+ * the linear that reads it in the same stream (quantize, then run something else or synchronise, then
+ * multiply).  It pays in launch-bound sequences: a decode step is ~130 kernels of 3-17 us. */
 SGQ_API int sgq_set_stream_overlap(int enabled);
 
 /* Kernels that wait on hardware barriers (TMA / tensor-core pipelines) bound every wait; one that
@@ -147,7 +148,8 @@ SGQ_API int sgq_codes_from_f32_int4(const float* codes_f32, int64_t numel, uint8
 
 /* Bytes of scratch the forward wants for this shape and path (0 = none).  bits is 4 or 8.  With SGQ_PATH_AUTO:
  * enough for whichever path AUTO takes - the decode kernels up to 16 rows, blocks of 16 rows on the decode kernels
- * up to 63 rows (the blocks share the scratch), the tensor-core path from 64 rows on. */
+ * up to 63 rows (INT4 stored [N,K]: converted activations of all blocks; else the blocks share one block's
+ * scratch, which is also what INT4 runs on when it gets no more), the tensor-core path from 64 rows on. */
 SGQ_API size_t sgq_linear_workspace_bytes(int bits, int64_t M, int64_t K, int64_t N, int layout, int path);
 
 /* Replaces quantization::quantized_matmul_int4 (src/quantization.cpp:199-206), i.e.

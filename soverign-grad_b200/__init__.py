@@ -131,8 +131,8 @@ def check(status: int, what: str = "sgq call") -> None:
 
 
 def set_stream_overlap(enabled) -> int:
-    """Programmatic dependent launch for every kernel of the library (see sgq_set_stream_overlap in
-    include/sgq.h for the one rule it adds).  Returns the previous setting."""
+    """1: decode kernels may fetch weights before older kernels in the stream are complete (sgq_set_stream_overlap in
+    include/sgq.h has the one rule that adds); 2: the two-CTAs-per-SM form as well; 0: off.  Returns the previous setting."""
     return int(lib.sgq_set_stream_overlap(int(enabled)))
 
 

@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kThreads) quantize_int8_rows_scalar_kernel(con
 // Compulsory bytes per element: 4 read + 1 written; 8 read + 1 written when the tensor does
 // not stay in L2 between steps 2 and 3.
 // ------------------------------------------------------------------------------------------
-// The four kernels of this path are launched with programmatic stream serialization when overlap is on: each lets
-// the next one start its launch and waits for the one before it before it touches the cell or the tensor.
+// The four kernels of this path are launched with programmatic stream serialization: each lets the next one start
+// its launch and waits for the one before it before it touches the cell or the tensor.
 __global__ void set_f32_kernel(float* p, float v) {
     pdl_launch_dependents();
     pdl_wait();

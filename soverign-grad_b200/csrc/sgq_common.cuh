@@ -44,9 +44,9 @@ struct SmemOptIn {
     }
 };
 
-// Process-wide switch (sgq_set_stream_overlap): kernels are launched with programmatic stream
-// serialization, so that a kernel's prologue, and for the decode kernel its first weight tiles,
-// overlap the tail of the kernel before it in the stream.
+// Process-wide switch (sgq_set_stream_overlap): the decode kernels may fetch their first weight tiles, and the
+// conversion kernels in front of them let them start, before older kernels in the stream are complete.  (The launch
+// attribute does not depend on it, see launch_kernel's callers: every kernel waits before it touches another's data.)
 bool stream_overlap_enabled();
 bool stream_overlap_compact();     // mode 2: the decode kernel also takes its two-CTAs-per-SM form
 

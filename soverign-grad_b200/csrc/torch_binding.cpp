@@ -1,5 +1,5 @@
 // Native side of the Python package's hot calls: takes torch tensors and the package's own objects, allocates the
-// outputs, and calls the C ABI of include/sgq.h — the same checks and results as the Python code it replaces.
+// outputs, and calls the C ABI of include/sgq.h.
 //
 // Why it exists: a decode-sized forward takes 5-10 us on the GPU, and the Python form of the call (attribute walks,
 // contiguous / float checks, a ctypes call with sixteen converted arguments, the stream lookup) took 15-20 us on the

@@ -152,8 +152,8 @@ class NanoLlamaInt4:
         self.cfg, self.device, self.batch = cfg, torch.device(device), batch
         self.rank, self.world, self.group = rank, world, group
         self.decode_path, self.prefill_path = decode_path, prefill_path
-        # consecutive kernels overlap (sgq_set_stream_overlap): legal here because no weight is ever
-        # written by the kernel in front of the linear that reads it
+        # weights may be fetched before older kernels are complete (sgq_set_stream_overlap): legal here because no
+        # weight is ever written by the kernel in front of the linear that reads it
         self.overlap = overlap
         # world > 1, decode steps: "peer" = slices stored into every rank's buffers by this library's kernels +
         # sgq_peer_barrier (graph-capturable); "nccl" = all-gather + interleave (eager).  A prompt pass of fewer
