@@ -243,7 +243,7 @@ gemv_int8_nk_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     // ---------------- consumers ----------------
     pdl_wait();                                     // the planes are the output of the conversion kernel
-    const int g = lane >> 2, t = lane & 3;
+    const int t = lane & 3;
     const int my_tile = warp % RT, sis = warp / RT;      // tile of the block, step inside the stage
     // ldmatrix row address of this lane inside a step box for group i (bytes 32 i .. 32 i + 31 of every row):
     // matrix (lane >> 3) = (rows 0-7 | rows 8-15) x (16-byte chunk 2i | 2i+1); 128-byte swizzle: chunk ^ (row & 7)
@@ -392,12 +392,14 @@ struct Plan {
     size_t planes_bytes;
 };
 
-// Tiles per block: as many as a CTA has at most, up to four.  N <= 0: any (support and workspace do not depend on it).
+// Tiles per block: as many as a CTA has at most, up to four; but two tiles one at a time from nine rows on (three column
+// sets), where a stage of two tiles and their planes leaves room for two stages only: [4096,4096] 12 rows 11.1 us in blocks
+// of two, 8.8 so, 16 rows 12.1 and 9.8; eight rows 9.0 either way.  N <= 0: any (support and workspace do not depend on it).
 bool make_plan(int64_t M, int64_t K, int64_t N, Plan* p) {
     p->L = prepared_layout(M, K);
     p->planes_bytes = p->L.bytes;
     const int64_t most = N > 0 ? ceil_div(ceil_div(N, kRows), sm_count()) : 1;
-    p->rt = most >= 3 ? 4 : (most == 2 ? 2 : 1);
+    p->rt = most >= 3 ? 4 : (most == 2 && p->L.nmain <= 2 ? 2 : 1);
     for (int st = kMaxStages; st >= 2; --st) {
         const Smem S = smem_layout(st, p->L.nmain, p->L.nlow, p->rt);
         if (S.total + 1024 <= static_cast<uint32_t>(kSmemLimit)) {
@@ -427,7 +429,9 @@ template <int NM, int NL, int MODE>
 int launch_variant(const LinearArgs& a, const Plan& p, const CUtensorMap& map_w, const CUtensorMap& map_block, int grid) {
     switch (p.rt) {
         case 1: return launch_blocks<NM, NL, MODE, 1>(a, p, map_w, map_block, grid);
-        case 2: return launch_blocks<NM, NL, MODE, 2>(a, p, map_w, map_block, grid);
+        case 2:
+            if constexpr (NM <= 2) return launch_blocks<NM, NL, MODE, 2>(a, p, map_w, map_block, grid);
+            [[fallthrough]];
         default: return launch_blocks<NM, NL, MODE, 4>(a, p, map_w, map_block, grid);
     }
 }

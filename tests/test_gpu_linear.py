@@ -146,8 +146,9 @@ def test_decode_int8_kernel_against_port(sgq, port, M, K, N):
     assert err.value.status == 5
 
 
-# (N / 16 tiles over 148 SMs: up to two tiles per CTA are worked on in blocks of two, from three on in blocks of four)
-TILE_BLOCKS_I8 = [(1, 1024, 2601), (16, 4224, 2601), (4, 8192, 4735), (2, 1152, 4999), (5, 2176, 5003), (7, 128, 4737), (9, 1664, 7217),
+# (N / 16 tiles over 148 SMs: two tiles per CTA are worked on in blocks of two up to eight rows and one by one from nine on,
+# three and more in blocks of four)
+TILE_BLOCKS_I8 = [(1, 1024, 2601), (8, 1920, 4601), (9, 1152, 4735), (16, 4224, 2601), (4, 8192, 4735), (2, 1152, 4999), (5, 2176, 5003), (7, 128, 4737), (9, 1664, 7217),
                   (12, 640, 9491), (15, 1280, 14001), (3, 1408, 11008)]
 
 
